@@ -519,7 +519,11 @@ void stage_t(int krk, double dt1) {
   }
   if (NS > 1) {
     KTimer t(KC_TRANSPORT);
-    k_transport<NS><<<nblk(N, 32), dim3(32, NS), 0, L->st>>>(L->d, L->T, L->p, L->di, L->amu, L->amk, L->amd);
+    const DevConst& c = L->hc;
+    if (c.flag_vis != 0 && c.flag_cond != 0 && c.flag_diff != 0)  // every property from its fit (Wilke)
+      launch_transport_fit(NS, N, L->T, L->p, L->di, L->amu, L->amk, L->amd, L->st);
+    else
+      k_transport<NS><<<nblk(N, 32), dim3(32, NS), 0, L->st>>>(L->d, L->T, L->p, L->di, L->amu, L->amk, L->amd);
     LAUNCH_CHECK();
   }
   {
@@ -1509,6 +1513,7 @@ int ocfd_gpu_init(const ocfd_params* p, const ocfd_thermo* th, const ocfd_kineti
     for (int m = 0; m < 3; m++) c.mass_force[m] = p->mass_force[m];
     fill_thermo(c, th, p->if_realgas);
     fill_trans(c, tr, p->n_spec);
+    CK(transport_fit_setup(c, p->n_spec));
     c.timeadv = p->chem_timeadv;
     if (kin) {
       if (kin->n_spec != p->n_spec || kin->n_reac > OCFD_MAX_REAC) { g_err = "kinetics size"; return OCFD_ERR_PARAM; }

@@ -29,6 +29,11 @@ void launch_chem_cells(int ns, long long ncell, double* f, double* Et, double* T
                        int nsub, int* nfail, cudaStream_t st);
 void launch_chem_batch(int ns, int sms, int n, double* di, double* e, const double* dt, const int* nsub,
                        const int* perm, int* counter, int* nfail, cudaStream_t st);
+// fitted mixture transport (Flag_vis = Flag_cond = Flag_diff = 1, N_SPEC 2..9; ocfd_transport.cu);
+// the set-up fills its constants and is not for stream capture
+cudaError_t transport_fit_setup(const DevConst& c, int ns);
+void launch_transport_fit(int ns, long long N, const double* T, const double* p, const double* di, double* amu,
+                          double* amk, double* amd, cudaStream_t st);
 // the compiled mechanism whose structure the constant block's mechanism has (MECH_H2AIR9), else
 // MECH_GENERIC (ocfd_chem.cu)
 int mech_match(const DevConst& c);
