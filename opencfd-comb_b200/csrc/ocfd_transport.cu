@@ -7,13 +7,13 @@
 #include <stdexcept>
 
 #include "ocfd_device.cuh"
+#include "ocfd_exp2.cuh"
 #include "ocfd_launch.h"
 
 namespace ocfd {
 
 // ---------------------------------------------------------------- constants of the fits
 constexpr int TF_NS = 9, TF_NP = TF_NS * (TF_NS - 1) / 2;
-constexpr int E2_N = 64;  // entries of the 2^(j / 64) table
 struct TransFit {
   // base-2 exponents of sqrt(mu_k), kappa_k and 1 / D_ab as cubics in ln T (the unit factors of the
   // fits folded into the constant term); pairs (a, b), a < b, enumerated a-major
@@ -23,7 +23,6 @@ struct TransFit {
   double rMi[TF_NS];
 };
 __constant__ TransFit cF;
-__device__ double g_exp2_tab[E2_N];
 
 // Fills the constants for the current set-up; called by ocfd_gpu_init, outside any capture.
 cudaError_t transport_fit_setup(const DevConst& c, int ns) {
@@ -49,40 +48,11 @@ cudaError_t transport_fit_setup(const DevConst& c, int ns) {
         t.dif[np][m] = (double)(-log2e * c.d_an[k][b][m] + (m == 0 ? std::log2(1.0e4L) : 0.0L));
     t.rMi[k] = 1.0 / c.Mi[k];
   }
-  double tab[E2_N];
-  for (int j = 0; j < E2_N; j++) tab[j] = (double)std::exp2((long double)j / E2_N);
-  cudaError_t e = cudaMemcpyToSymbol(cF, &t, sizeof(t));
-  return e != cudaSuccess ? e : cudaMemcpyToSymbol(g_exp2_tab, tab, sizeof(tab));
+  const cudaError_t e = cudaMemcpyToSymbol(cF, &t, sizeof(t));
+  return e != cudaSuccess ? e : exp2_tab_setup();
 }
 
 // ---------------------------------------------------------------- arithmetic
-// 1 / x for normal x: the hardware's approximation (about 2^-23) refined by one third-order Newton
-// (Householder) step, y (1 + e + e^2) with e = 1 - x y, whose error term e^3 is below the last place
-__device__ __forceinline__ double rcp3(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-// 2^y by table and polynomial (P. T. P. Tang, "Table-driven implementation of the exponential
-// function in IEEE floating-point arithmetic", ACM TOMS 15, 1989): y = n / 64 + r, |r| <= 1 / 128,
-// 2^y = 2^(n >> 6) tab[n & 63] 2^r with the Taylor polynomial of degree 5 (remainder 4e-17). Nine
-// FP64 operations; the binary exponent is added as an integer and saturates at the normal range.
-__device__ __forceinline__ double exp2_tab(double y, const double* tab) {
-  constexpr double MAGIC = 6755399441055744.0;  // 1.5 2^52: the sum's low word is rint(64 y)
-  const double t = fma(y, (double)E2_N, MAGIC);
-  const double nf = t - MAGIC;
-  const double r = fma(nf, -1.0 / E2_N, y);
-  const int n = __double2loint(t);
-  constexpr double L1 = 0.69314718055994530942;
-  constexpr double c1 = L1, c2 = L1 * L1 / 2, c3 = L1 * L1 * L1 / 6, c4 = L1 * L1 * L1 * L1 / 24,
-                   c5 = L1 * L1 * L1 * L1 * L1 / 120;
-  const double q = fma(r, fma(r, fma(r, fma(r, c5, c4), c3), c2), c1) * r;
-  const double tv = tab[n & (E2_N - 1)];
-  const int ex = max(min(n >> 6, 1022), -1022);
-  const double s = __hiloint2double(__double2hiint(tv) + (ex << 20), __double2loint(tv));
-  return fma(s, q, s);
-}
 __device__ __forceinline__ double cubic(const double* c, double L) {
   return fma(fma(fma(c[3], L, c[2]), L, c[1]), L, c[0]);
 }
@@ -106,7 +76,7 @@ __global__ void __launch_bounds__(OCFD_TFIT_THREADS, OCFD_TFIT_MINB)
     k_transport_fit(const double* __restrict__ T, const double* __restrict__ p, const double* __restrict__ di,
                     double* __restrict__ amu, double* __restrict__ amk, double* __restrict__ amd) {
   __shared__ double tab[E2_N];
-  if (threadIdx.x < E2_N) tab[threadIdx.x] = g_exp2_tab[threadIdx.x];
+  exp2_tab_load(tab);
   __syncthreads();
   const unsigned t = blockIdx.x * OCFD_TFIT_THREADS + threadIdx.x;
   if (t >= (unsigned)cC.N) return;
