@@ -247,7 +247,8 @@ int ocfd_gpu_chem_constant_pressure(int on);
  * (opencfd-comb_b200/csrc/ocfd_mech_h2air9.cuh, generated from its data file). When the loaded
  * mechanism has exactly that structure (species count, reactions, stoichiometry, rate forms,
  * third-body flags) and CHEM_TimeAdv = -1, the flow step's chemistry and the batched reactors
- * run it; its numbers equal the generic kernels' bit for bit on finite states. on = 0 keeps the
+ * run it; its numbers equal the generic kernels' bit for bit on finite states (in the contracted
+ * build up to rounding). on = 0 keeps the
  * generic kernels, on = 1 allows the compiled ones (default), on < 0 changes nothing. Returns 1
  * when the compiled kernels are in use for the current set-up, else 0. */
 int ocfd_gpu_chem_compiled_mechanism(int on);

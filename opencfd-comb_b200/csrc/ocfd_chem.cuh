@@ -449,14 +449,28 @@ static __global__ void k_nsub_hist(int n, const int* nsub, int* hist, int nbins)
   int b = min(max(s, 0), nbins - 1);
   atomicAdd(&hist[nbins - 1 - b], 1);  // descending sub-step count
 }
+// exclusive prefix sums of the histogram, one block of nbins threads (a warp scan of warp totals)
 static __global__ void k_nsub_scan(int* hist, int nbins) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int acc = 0;
-  for (int b = 0; b < nbins; b++) {
-    int c = hist[b];
-    hist[b] = acc;
-    acc += c;
+  __shared__ int tot[32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int c = t < nbins ? hist[t] : 0;
+  int x = c;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
   }
+  if (lane == 31) tot[w] = x;
+  __syncthreads();
+  if (w == 0) {
+    int s = lane < (int)(blockDim.x >> 5) ? tot[lane] : 0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += y;
+    }
+    tot[lane] = s;
+  }
+  __syncthreads();
+  if (t < nbins) hist[t] = x - c + (w > 0 ? tot[w - 1] : 0);
 }
 static __global__ void k_nsub_scatter(int n, const int* nsub, int* cursor, int nbins, int* perm) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;

@@ -1518,6 +1518,7 @@ int ocfd_gpu_init(const ocfd_params* p, const ocfd_thermo* th, const ocfd_kineti
     if (kin) {
       if (kin->n_spec != p->n_spec || kin->n_reac > OCFD_MAX_REAC) { g_err = "kinetics size"; return OCFD_ERR_PARAM; }
       fill_kin(c, kin);
+      CK(mech_setup(c));
       L->have_kin = true;
     }
     CK(cudaMemcpyToSymbol(cC, &c, sizeof(DevConst)));
@@ -2109,6 +2110,7 @@ int ocfd_gpu_chem_setup(const ocfd_thermo* th, const ocfd_kinetics* kin, int rea
     L->hc.timeadv = timeadv;
     L->hc.ns = th->n_spec;
     L->hc.const_p = 0;  // the reference's constant-volume reactor unless ocfd_gpu_chem_constant_pressure(1)
+    CK(mech_setup(L->hc));
     L->have_kin = true;
     CK(cudaMemcpyToSymbol(cC, &L->hc, sizeof(DevConst)));
     return 0;
@@ -2136,7 +2138,7 @@ int ocfd_gpu_chem_batch_device(int n, double* d_di, double* d_e, const double* d
     {
       KTimer t(KC_CHEM);
       k_nsub_hist<<<nblk(n, 256), 256, 0, L->st>>>(n, d_nsub, L->b_hist, nbins);
-      k_nsub_scan<<<1, 32, 0, L->st>>>(L->b_hist, nbins);
+      k_nsub_scan<<<1, nbins, 0, L->st>>>(L->b_hist, nbins);
       k_nsub_scatter<<<nblk(n, 256), 256, 0, L->st>>>(n, d_nsub, L->b_hist, nbins, L->b_perm);
       LAUNCH_CHECK();
     }
@@ -2216,7 +2218,7 @@ int ocfd_gpu_chem_batch_noalloc(int n, double* d_di, double* d_e, const double* 
     {
       KTimer t(KC_CHEM);
       k_nsub_hist<<<nblk(n, 256), 256, 0, L->st>>>(n, d_nsub, hist, OCFD_NOALLOC_BINS);
-      k_nsub_scan<<<1, 32, 0, L->st>>>(hist, OCFD_NOALLOC_BINS);
+      k_nsub_scan<<<1, OCFD_NOALLOC_BINS, 0, L->st>>>(hist, OCFD_NOALLOC_BINS);
       k_nsub_scatter<<<nblk(n, 256), 256, 0, L->st>>>(n, d_nsub, hist, OCFD_NOALLOC_BINS, perm);
       LAUNCH_CHECK();
     }

@@ -37,4 +37,7 @@ void launch_transport_fit(int ns, long long N, const double* T, const double* p,
 // the compiled mechanism whose structure the constant block's mechanism has (MECH_H2AIR9), else
 // MECH_GENERIC (ocfd_chem.cu)
 int mech_match(const DevConst& c);
+// constants of the compiled mechanism's contracted-build step, when the tables match it (not for
+// stream capture)
+cudaError_t mech_setup(const DevConst& c);
 }  // namespace ocfd
