@@ -869,9 +869,10 @@ __global__ void __launch_bounds__(VE_THREADS, 2) k_visc_div(DivArgs a) {
   }
 }
 
-// resident-block target of the per-cell k_visc_div: it waits on its stencil loads, so a fifth
-// block per SM (48 registers, about 20 bytes spilled to L1) measured 4 % faster than four (55
-// registers); six (40 registers, 50 bytes spilled) gained nothing
+// resident-block target of the per-cell k_visc_div: it waits on its stencil loads; ten blocks of 128
+// threads (48 registers) against eight / twelve: 1.126 against 1.158 / 1.098 ms per step on the
+// 384x256x32 jet, 0.201 against 0.223 / 0.210 on 97x61x43, 1.55 against 1.55 / 1.58 on 1024x160x32.
+// In 32 x 4 tiles of cells: on those grids 1.69 (marching, 16 planes), 0.52 and 2.37 ms per step
 #ifndef OCFD_VDIV_MINB
 #define OCFD_VDIV_MINB 5
 #endif
@@ -920,6 +921,60 @@ static __global__ void k_ci(const double* di, const double* d, double* ci, long 
   const size_t o = (size_t)blockIdx.y * H;
   if (t < H) ci[o + t] = di[o + t] / d[t];
 }
+// Cells within E layers of the non-periodic faces, enumerated: the x slabs, the y slabs without them,
+// the z slabs without both. n = 0 everywhere for a fully periodic grid.
+struct Shell {
+  int lo[3], hi[3];          // first and last index of the core along each direction
+  long long nxs, nys, nzs;   // cells of the three groups of slabs
+  __host__ long long count() const { return nxs + nys + nzs; }
+};
+static inline Shell make_shell(const int* n, const int* iper, int e) {
+  Shell s{};
+  long long c[3], o[3];
+  for (int d = 0; d < 3; d++) {
+    const int l = iper[d] ? 0 : e;
+    s.lo[d] = 1 + l;
+    s.hi[d] = n[d] - l;
+    if (s.hi[d] < s.lo[d] - 1) s.hi[d] = s.lo[d] - 1;  // thin grid: everything is shell
+    c[d] = s.hi[d] - s.lo[d] + 1;
+    o[d] = n[d] - c[d];
+  }
+  s.nxs = o[0] * n[1] * (long long)n[2];
+  s.nys = c[0] * o[1] * (long long)n[2];
+  s.nzs = c[0] * c[1] * o[2];
+  return s;
+}
+__device__ __forceinline__ int shell_out(const Shell& s, int d, int t) {  // t-th index outside the core
+  return t < s.lo[d] - 1 ? t + 1 : s.hi[d] + 1 + (t - (s.lo[d] - 1));
+}
+__device__ __forceinline__ bool shell_cell(const Shell& s, long long t64, int& i, int& j, int& k) {
+  if (t64 >= s.nxs + s.nys + s.nzs) return false;
+  unsigned t = (unsigned)t64;
+  if (t64 < s.nxs) {
+    const unsigned o = (unsigned)(cC.nx - (s.hi[0] - s.lo[0] + 1));
+    i = shell_out(s, 0, (int)(t % o));
+    t /= o;
+    j = (int)(t % (unsigned)cC.ny) + 1;
+    k = (int)(t / (unsigned)cC.ny) + 1;
+    return true;
+  }
+  t -= (unsigned)s.nxs;
+  const unsigned cx = (unsigned)(s.hi[0] - s.lo[0] + 1);
+  i = s.lo[0] + (int)(t % cx);
+  unsigned r = t / cx;
+  if (t < (unsigned)s.nys) {
+    const unsigned o = (unsigned)(cC.ny - (s.hi[1] - s.lo[1] + 1));
+    j = shell_out(s, 1, (int)(r % o));
+    k = (int)(r / o) + 1;
+    return true;
+  }
+  r = (t - (unsigned)s.nys) / cx;
+  i = s.lo[0] + (int)((t - (unsigned)s.nys) - r * cx);
+  const unsigned cy = (unsigned)(s.hi[1] - s.lo[1] + 1);
+  j = s.lo[1] + (int)(r % cy);
+  k = shell_out(s, 2, (int)(r / cy));
+  return true;
+}
 // One thread per (cell, species): a block is 32 consecutive cells (threadIdx.x) x NS species
 // (threadIdx.y), so every species' loads are coalesced and the NS stencil evaluations of a cell
 // run in parallel. The enthalpy-flux sums Qp go through shared memory and are added by the
@@ -931,14 +986,17 @@ static __global__ void k_ci(const double* di, const double* d, double* ci, long 
 #ifndef OCFD_SPECIES_MINB
 #define OCFD_SPECIES_MINB 3
 #endif
+// SEP: the face cells of a tensor-product grid (sh), else every cell of a general grid (k_spec_ev, in
+// ocfd_species.cu, has the rest)
 template <int NS, bool SEP>
 __global__ void __launch_bounds__(32 * NS, OCFD_SPECIES_MINB) k_scal_ev(const double* ci, const double* d, const double* T,
                                                      const double* amd, double* qpx, double* qpy, double* qpz,
-                                                     double* e1, double* e2, double* e3, Geo g) {
+                                                     double* e1, double* e2, double* e3, Geo g, Shell sh = {}) {
   __shared__ double sq[3][NS][32];
   const int ks = threadIdx.y, lane = threadIdx.x;
   int i, j, k;
-  const bool ok = cell_of_slab((long long)blockIdx.x * 32 + lane, i, j, k);
+  const long long t = (long long)blockIdx.x * 32 + lane;
+  const bool ok = SEP ? shell_cell(sh, t, i, j, k) : cell_of_slab(t, i, j, k);
   int nn = 0;
   if (ok) {
     const int q = hidx(i, j, k);
@@ -988,15 +1046,16 @@ __global__ void __launch_bounds__(32 * NS, OCFD_SPECIES_MINB) k_scal_ev(const do
 #endif
 // RK: the species RK update (k_scal_rk's expressions on the finished Dus value, which then stays in
 // a register instead of making a round trip through HBM; nothing else reads Dus afterwards)
-template <int NS, bool SEP, bool RK = false>
+template <int NS, bool SEP, bool RK>
 __global__ void __launch_bounds__(32 * NS, OCFD_SCAL_DIV_MINB) k_scal_div(const double* e1, const double* e2,
                                                                           const double* e3, double* dus, Geo g,
-                                                                          int krk = 0, double dt = 0.0,
-                                                                          const double* din = nullptr,
-                                                                          double* di = nullptr) {
+                                                                          int krk, double dt,
+                                                                          const double* din,
+                                                                          double* di, Shell sh = {}) {
   const int ks = threadIdx.y;
   int i, j, k;
-  const bool ok = cell_of_slab((long long)blockIdx.x * 32 + threadIdx.x, i, j, k);
+  const long long t = (long long)blockIdx.x * 32 + threadIdx.x;
+  const bool ok = SEP ? shell_cell(sh, t, i, j, k) : cell_of_slab(t, i, j, k);
   if (!ok) return;
   const int q = hidx(i, j, k), nn = nidx(i, j, k);
   const double jac = metric_jac<SEP>(g, i, j, k, q);  // every species' thread (no barrier)

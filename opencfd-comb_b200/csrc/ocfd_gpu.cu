@@ -575,7 +575,14 @@ void stage_rhs_t(int krk, double dt1, bool rk) {
     }
     std::swap(L->st, L->st3);
   };
-  const bool sp_visc = NS > 1 && L->P.if_viscous == 1;
+  const bool sp_visc = NS > 1 && L->P.if_viscous == 1, cd8 = L->P.scheme_vis == OCFD_SCHEME_CD8;
+  SpecArgs sa{};
+  sa.ci = L->ci; sa.d = L->d; sa.T = L->T; sa.amd = L->amd; sa.din = L->din; sa.dus = L->dus; sa.di = L->di;
+  for (int m = 0; m < 3; m++) { sa.qp[m] = L->qp[m]; sa.se[m] = L->se[m]; }
+  sa.g = L->geo;
+  sa.nx = L->P.nx; sa.ny = L->P.ny; sa.nz = L->P.nz;
+  const int ncell[3] = {L->P.nx, L->P.ny, L->P.nz};
+  const Shell shell = make_shell(ncell, L->P.iperiodic, face_layers(cd8));
   auto species_sweeps = [&]() {
     const int grp = NS % 3 == 0 ? 3 : 1;
     FluxArgs fs = fa;
@@ -584,22 +591,22 @@ void stage_rhs_t(int krk, double dt1, bool rk) {
     for (int dd = 0; dd < 3; dd++) launch_flux(dd, fs, grp, NS / grp);
   };
   auto species_div_rk = [&]() {
-    if (sp_visc && rk) {  // the divergence with the species RK update fused in
+    if (sp_visc) {  // the divergence, with rk the species RK update fused in
       KTimer t(KC_SPECIES_VISC);
-      if (L->sep)
-        k_scal_div<NS, true, true><<<nblk(N, 32), dim3(32, NS), 0, L->st>>>(L->se[0], L->se[1], L->se[2], L->dus,
-                                                                          L->geo, krk, dt1, L->din, L->di);
-      else
-        k_scal_div<NS, false, true><<<nblk(N, 32), dim3(32, NS), 0, L->st>>>(L->se[0], L->se[1], L->se[2], L->dus,
-                                                                           L->geo, krk, dt1, L->din, L->di);
-      LAUNCH_CHECK();
-      return;
-    }
-    if (sp_visc) {
-      KTimer t(KC_SPECIES_VISC);
-      if (L->sep) k_scal_div<NS, true><<<nblk(N, 32), dim3(32, NS), 0, L->st>>>(L->se[0], L->se[1], L->se[2], L->dus, L->geo);
-      else k_scal_div<NS, false><<<nblk(N, 32), dim3(32, NS), 0, L->st>>>(L->se[0], L->se[1], L->se[2], L->dus, L->geo);
-      LAUNCH_CHECK();
+      if (L->sep) {
+        launch_spec_div(NS, cd8, rk ? krk : 0, dt1, sa, L->st);
+        LAUNCH_CHECK();
+      }
+      const unsigned nb = nblk(L->sep ? shell.count() : N, 32);
+      auto div = [&](auto kern) {
+        kern<<<nb, dim3(32, NS), 0, L->st>>>(L->se[0], L->se[1], L->se[2], L->dus, L->geo, krk, dt1, L->din, L->di, shell);
+        LAUNCH_CHECK();
+      };
+      if (nb > 0) {
+        if (L->sep) rk ? div(k_scal_div<NS, true, true>) : div(k_scal_div<NS, true, false>);
+        else rk ? div(k_scal_div<NS, false, true>) : div(k_scal_div<NS, false, false>);
+      }
+      if (rk) return;
     }
     if (rk) {
       KTimer t(KC_SPECIES_RK);
@@ -620,8 +627,16 @@ void stage_rhs_t(int krk, double dt1, bool rk) {
         KTimer t(KC_SPECIES_VISC);
         k_ci<<<dim3(nblk(H, 256), NS), 256, 0, L->st>>>(L->di, L->d, L->ci, H);
         LAUNCH_CHECK();
-        if (L->sep) k_scal_ev<NS, true><<<nblk(N, 32), dim3(32, NS), 0, L->st>>>(L->ci, L->d, L->T, L->amd, L->qp[0], L->qp[1], L->qp[2], L->se[0], L->se[1], L->se[2], L->geo);
-        else k_scal_ev<NS, false><<<nblk(N, 32), dim3(32, NS), 0, L->st>>>(L->ci, L->d, L->T, L->amd, L->qp[0], L->qp[1], L->qp[2], L->se[0], L->se[1], L->se[2], L->geo);
+        if (L->sep) {
+          launch_spec_ev(NS, cd8, sa, L->st);
+          LAUNCH_CHECK();
+        }
+        const unsigned nb = nblk(L->sep ? shell.count() : N, 32);
+        auto ev = [&](auto kern) {
+          kern<<<nb, dim3(32, NS), 0, L->st>>>(L->ci, L->d, L->T, L->amd, L->qp[0], L->qp[1], L->qp[2], L->se[0],
+                                              L->se[1], L->se[2], L->geo, shell);
+        };
+        if (nb > 0) L->sep ? ev(k_scal_ev<NS, true>) : ev(k_scal_ev<NS, false>);
         LAUNCH_CHECK();
       }
       for (int dd = 0; dd < 3; dd++) {
@@ -1514,6 +1529,7 @@ int ocfd_gpu_init(const ocfd_params* p, const ocfd_thermo* th, const ocfd_kineti
     fill_thermo(c, th, p->if_realgas);
     fill_trans(c, tr, p->n_spec);
     CK(transport_fit_setup(c, p->n_spec));
+    CK(species_setup(c, p->n_spec));
     c.timeadv = p->chem_timeadv;
     if (kin) {
       if (kin->n_spec != p->n_spec || kin->n_reac > OCFD_MAX_REAC) { g_err = "kinetics size"; return OCFD_ERR_PARAM; }

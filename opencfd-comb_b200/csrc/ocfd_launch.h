@@ -34,6 +34,18 @@ void launch_chem_batch(int ns, int sms, int n, double* di, double* e, const doub
 cudaError_t transport_fit_setup(const DevConst& c, int ns);
 void launch_transport_fit(int ns, long long N, const double* T, const double* p, const double* di, double* amu,
                           double* amk, double* amd, cudaStream_t st);
+// species viscous terms on tensor-product grids (ocfd_species.cu); krk = 1..3 runs the species RK
+// update on the finished Dus value, krk = 0 writes Dus back
+struct SpecArgs {
+  const double *ci, *d, *T, *amd, *din;
+  double *qp[3], *se[3], *dus, *di;
+  Geo g;
+  int nx, ny, nz;
+};
+cudaError_t species_setup(const DevConst& c, int ns);  // constants; not for stream capture
+int face_layers(bool cd8);  // cells this near a non-periodic face are left to k_scal_ev / k_scal_div
+void launch_spec_ev(int ns, bool cd8, const SpecArgs& a, cudaStream_t st);
+void launch_spec_div(int ns, bool cd8, int krk, double dt, const SpecArgs& a, cudaStream_t st);
 // the compiled mechanism whose structure the constant block's mechanism has (MECH_H2AIR9), else
 // MECH_GENERIC (ocfd_chem.cu)
 int mech_match(const DevConst& c);
