@@ -315,7 +315,9 @@ int ocfd_gpu_ana_average(int upload, double* fields, int* k_average, double* t_a
  * the viscous flux after and beside the flux sweeps, then a stage's right-hand sides without the
  * species RK update with the species chain in order and on the third stream (-1 where not timed).
  * The launches write only scratch arrays, so the solution is unchanged. Default choice
- * {0, 0, 0, 16, 16, 0, 0, 0, 3}. */
+ * {0, 0, 0, 16, 16, 0, 0, 0, 3}, with the two viscous kernels in their per-cell forms until a choice
+ * is set or tuned; the tuner also times the per-cell k_visc_ev (not among the 27 times) and keeps it
+ * where it is the fastest. */
 int ocfd_gpu_autotune(int reps, int* choice, double* ms);
 int ocfd_gpu_set_tiles(const int* choice);
 int ocfd_gpu_get_tiles(int* choice);

@@ -571,6 +571,23 @@ __device__ __forceinline__ bool cell_of_slab(long long t64, int& i, int& j, int&
   return true;
 }
 
+// the cell of a thread in blocks of a 32 x PC_TY tile of one plane; the blocks of a slab of 32 rows
+// walk all planes before the next slab, so that z neighbours are read again while L2 holds them.
+// Grid: (tiles in i x tiles of a slab, nz, slabs) (pc_grid)
+constexpr int PC_TY = 4, PC_SLAB = 32 / PC_TY;
+__device__ __forceinline__ bool cell_of_tile(int nbx, int& i, int& j, int& k) {
+  const int bx = (int)blockIdx.x % nbx, bj = (int)blockIdx.x / nbx;
+  i = bx * 32 + (int)threadIdx.x % 32 + 1;
+  j = ((int)blockIdx.z * PC_SLAB + bj) * PC_TY + (int)threadIdx.x / 32 + 1;
+  k = (int)blockIdx.y + 1;
+  return i <= cC.nx && j <= cC.ny;
+}
+static inline dim3 pc_grid(int nx, int ny, int nz, int& nbx) {
+  nbx = (nx + 31) / 32;
+  const int nby = (ny + PC_TY - 1) / PC_TY;
+  return dim3((unsigned)(nbx * PC_SLAB), (unsigned)nz, (unsigned)((nby + PC_SLAB - 1) / PC_SLAB));
+}
+
 struct ViscArgs {
   const double *d, *u, *v, *w, *T, *di;
   const double *amu, *amk;        // precomputed transport (NS > 1) or nullptr
@@ -746,6 +763,41 @@ __global__ void __launch_bounds__(VE_THREADS, OCFD_VE_MINB) k_visc_ev(ViscArgs a
   }
 }
 
+// k_visc_ev with one thread per cell: every stencil value through the read-only cache, the same
+// expressions as the marching form. No serial walk through planes and no barrier: the marching form
+// needs a chunk of planes per block to pay for its halo, which leaves a small grid with a few long
+// blocks (16 planes one after another are 67 us per launch on a 16^3 grid), and at every size its
+// barriers and two resident blocks cost more than the gathers do. ms per step, marching at its
+// default 16 planes / at its best chunk / this form: 16^3 0.40 / 0.09 / 0.07; 64^3 0.43 / 0.18 / 0.17;
+// 81^3 CD8 0.81 / 0.56 / 0.32; 97x61x43 0.75 / 0.31 / 0.34; 384x256x32 2.04 / 1.87 / 1.66; 1024x160x32
+// 3.45 / 3.20 / 2.50. Six blocks (80 registers) hide the loads best: 1.78 and 2.02 ms at five and four
+// on the 384x256x32 grid.
+#ifndef OCFD_VEPC_MINB
+#define OCFD_VEPC_MINB 6
+#endif
+template <int NS, bool SEP, int HZ>
+__global__ void __launch_bounds__(32 * PC_TY, OCFD_VEPC_MINB) k_visc_ev_pc(ViscArgs a, int nbx) {
+  constexpr int CD = HZ == 3 ? 6 : 8;
+  int i, j, k;
+  if (!cell_of_tile(nbx, i, j, k)) return;
+  const int q = hidx(i, j, k), sy = hstride(1), sz = hstride(2);
+  const double* fl[4] = {a.u, a.v, a.w, a.T};
+  double g[4][3];
+  if (cdiff_interior(0, i, cC.nx) && cdiff_interior(1, j, cC.ny) && cdiff_interior(2, k, cC.nz)) {
+#pragma unroll
+    for (int f = 0; f < 4; f++) cdiff3(fl[f], fl[f], fl[f], q, i, j, k, g[f][0], g[f][1], g[f][2]);
+  } else {
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+      const double* p = fl[f] + q;
+      g[f][0] = cdiff_g<CD>([&](int o) { return __ldg(p + o); }, 0, i, cC.nx);
+      g[f][1] = cdiff_g<CD>([&](int o) { return __ldg(p + o * sy); }, 1, j, cC.ny);
+      g[f][2] = cdiff_g<CD>([&](int o) { return __ldg(p + o * sz); }, 2, k, cC.nz);
+    }
+  }
+  visc_point<NS, SEP>(a, i, j, k, g, a.u[q], a.v[q], a.w[q], a.T[q]);
+}
+
 struct DivArgs {
   const double* ev[12];  // Ev1 (4), Ev2 (4), Ev3 (4) halo arrays, periodic halos exchanged
   double* du;
@@ -874,15 +926,15 @@ __global__ void __launch_bounds__(VE_THREADS, 2) k_visc_div(DivArgs a) {
 // 384x256x32 jet, 0.201 against 0.223 / 0.210 on 97x61x43, 1.55 against 1.55 / 1.58 on 1024x160x32.
 // In 32 x 4 tiles of cells: on those grids 1.69 (marching, 16 planes), 0.52 and 2.37 ms per step
 #ifndef OCFD_VDIV_MINB
-#define OCFD_VDIV_MINB 5
+#define OCFD_VDIV_MINB 10
 #endif
 // per-cell form of k_visc_div (the autotuner's k chunk 0): one thread per cell, every stencil
 // value read through the read-only cache; the same expressions as the marching form
 template <bool SEP, int HZ>
-__global__ void __launch_bounds__(256, OCFD_VDIV_MINB) k_visc_div_pc(DivArgs a) {
+__global__ void __launch_bounds__(32 * PC_TY, OCFD_VDIV_MINB) k_visc_div_pc(DivArgs a, int nbx) {
   constexpr int CD = HZ == 3 ? 6 : 8;
   int i, j, k;
-  if (!cell_of_slab((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+  if (!cell_of_tile(nbx, i, j, k)) return;
   const int q = hidx(i, j, k), nn = nidx(i, j, k);
   const int sy = hstride(1), sz = hstride(2);
   const long long N = cC.N;

@@ -115,6 +115,9 @@ struct Lib {
   // sweep direction, k planes per block of k_visc_ev and k_visc_div
   int flux_ts[3] = {0, 0, 0};
   int kc_ev = VE_KC, kc_div = VE_KC;
+  // the per-cell forms of the two viscous kernels instead of the marching ones: until a choice is
+  // set or tuned, and (k_visc_ev) when the tuner found it faster than every k chunk
+  bool ev_pc = true, div_pc = true;
   // metric form per kernel family on a tensor-product grid: false = computed from the 1-D
   // derivatives (separable), true = read from the 19 stored arrays (allocated on first use)
   bool met_flux = false, met_ev = false, met_div = false;
@@ -397,6 +400,12 @@ void visc_ev_go(const ViscArgs& va) {
     attr = true;
   }
   const ocfd_params& P = L->P;
+  if (va.kc == 0) {  // per-cell form
+    int nbx;
+    const dim3 grid = pc_grid(P.nx, P.ny, P.nz, nbx);
+    k_visc_ev_pc<NS, SEP, HZ><<<grid, 32 * PC_TY, 0, L->st>>>(va, nbx);
+    return;
+  }
   dim3 grid(nblk(P.nx, VE_TX), nblk(P.ny, VE_TY), nblk(P.nz, va.kc));
   k_visc_ev<NS, SEP, HZ><<<grid, VE_THREADS, sm, L->st>>>(va);
 }
@@ -411,7 +420,9 @@ void visc_div_go(const DivArgs& da) {
   }
   const ocfd_params& P = L->P;
   if (da.kc == 0) {  // per-cell form
-    k_visc_div_pc<SEP, HZ><<<nblk(L->hc.N, 256), 256, 0, L->st>>>(da);
+    int nbx;
+    const dim3 grid = pc_grid(P.nx, P.ny, P.nz, nbx);
+    k_visc_div_pc<SEP, HZ><<<grid, 32 * PC_TY, 0, L->st>>>(da, nbx);
     return;
   }
   dim3 grid(nblk(P.nx, VE_TX), nblk(P.ny, VE_TY), nblk(P.nz, da.kc));
@@ -437,7 +448,7 @@ ViscArgs visc_args() {
   for (int dd = 0; dd < 3; dd++)
     for (int m = 0; m < 4; m++) va.ev[dd][m] = L->ev[4 * dd + m];
   va.g = L->geo;
-  va.kc = L->kc_ev;
+  va.kc = L->ev_pc ? 0 : L->kc_ev;
   return va;
 }
 DivArgs div_args() {
@@ -445,7 +456,7 @@ DivArgs div_args() {
   for (int m = 0; m < 12; m++) da.ev[m] = L->ev[m];
   da.du = L->du;
   da.g = L->geo;
-  da.kc = L->kc_div;
+  da.kc = L->div_pc ? 0 : L->kc_div;
   return da;
 }
 template <int NS>
@@ -702,7 +713,7 @@ void chem_t(double dt2, int nsub) {
 // form computes), so the tuner is free to pick by time alone. Choices are remembered per
 // configuration in the process.
 constexpr int TUNE_N = 9, TUNE_TIMES = 3 * FLUX_TILE_SHAPES + 9 + 5 + 2 + 2;
-std::map<std::string, std::array<int, TUNE_N>> g_tune_cache;
+std::map<std::string, std::array<int, TUNE_N + 1>> g_tune_cache;  // the choice and best[TUNE_N]
 
 std::string tune_key() {
   const ocfd_params& P = L->P;
@@ -744,10 +755,12 @@ void ensure_stored_metrics() {
   set_geo_device_ptrs();
 }
 
-void apply_tiles(const int* c) {
+void apply_tiles(const int* c, bool ev_pc = false) {
   for (int d = 0; d < 3; d++) L->flux_ts[d] = c[d];
   L->kc_ev = c[3];
   L->kc_div = c[4];
+  L->ev_pc = ev_pc;
+  L->div_pc = false;  // c[4] = 0 names the per-cell form
   if (L->sep && (c[5] | c[6] | c[7])) ensure_stored_metrics();
   L->met_flux = c[5] != 0;
   L->met_ev = c[6] != 0;
@@ -761,7 +774,7 @@ void apply_tiles(const int* c) {
 // launches between two events) and applies the fastest; the launches write only scratch arrays
 // (du, Ev, the hybrid sensor) that every stage recomputes before it reads them
 template <int NS>
-void tune_t(int reps, int* best, double* ms) {
+void tune_t(int reps, int* best, double* ms) {  // best[TUNE_N]: k_visc_ev's per-cell form wins
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -796,6 +809,9 @@ void tune_t(int reps, int* best, double* ms) {
       L->flux_ts[d] = best[d];
     }
     best[3] = best[4] = VE_KC;
+    best[TUNE_N] = 0;
+    L->ev_pc = L->div_pc = false;
+    double t_evform = 1e300;  // k_visc_ev in the chosen form
     best[5] = best[6] = best[7] = L->sep ? 0 : 1;
     best[8] = NS > 1 ? 3 : 1;
     for (int m = 3 * FLUX_TILE_SHAPES; m < TUNE_TIMES; m++) ms[m] = -1.0;
@@ -807,6 +823,14 @@ void tune_t(int reps, int* best, double* ms) {
         const double t = timed([&] { visc_ev_launch<NS>(va); });
         ms[3 * FLUX_TILE_SHAPES + m] = t;
         if (t < t_ev) { t_ev = t; best[3] = va.kc; }
+      }
+      {
+        ViscArgs va = visc_args<NS>();
+        va.kc = 0;
+        const double t = timed([&] { visc_ev_launch<NS>(va); });
+        best[TUNE_N] = t < t_ev ? 1 : 0;
+        t_evform = std::min(t, t_ev);
+        L->ev_pc = best[TUNE_N] != 0;
       }
       for (int m = 0; m < 5; m++) {  // the four k chunks, then the per-cell form (0)
         DivArgs da = div_args();
@@ -836,12 +860,10 @@ void tune_t(int reps, int* best, double* ms) {
       if (P.if_viscous == 1) {
         L->met_ev = true;
         ViscArgs va = visc_args<NS>();
-        va.kc = best[3];
+        va.kc = L->ev_pc ? 0 : best[3];
         ms[M0 + 3] = timed([&] { visc_ev_launch<NS>(va); });
         L->met_ev = false;
-        int mi = 0;
-        for (int m = 0; m < 4; m++) if (VE_KC_CHOICES[m] == best[3]) mi = m;
-        best[6] = ms[M0 + 3] < ms[3 * FLUX_TILE_SHAPES + mi] ? 1 : 0;
+        best[6] = ms[M0 + 3] < t_evform ? 1 : 0;
         L->met_div = true;
         DivArgs da = div_args();
         da.kc = best[4];
@@ -2514,20 +2536,20 @@ int ocfd_gpu_autotune(int reps, int* choice, double* ms) {
   return guarded([&]() -> int {
     if (!L || !L->flow_ready) { g_err = "state not initialised"; return OCFD_ERR_STATE; }
     if (reps < 0) { g_err = "reps must be >= 0"; return OCFD_ERR_PARAM; }
-    int best[TUNE_N];
+    int best[TUNE_N + 1];
     double t[TUNE_TIMES];
     const std::string key = tune_key();
     auto it = g_tune_cache.find(key);
     if (reps == 0 && it != g_tune_cache.end()) {
-      for (int m = 0; m < TUNE_N; m++) best[m] = it->second[m];
+      for (int m = 0; m <= TUNE_N; m++) best[m] = it->second[m];
       for (int m = 0; m < TUNE_TIMES; m++) t[m] = -1.0;
     } else {
       NS_DISPATCH(L->NS, tune_t<NSV>(reps > 0 ? reps : 3, best, t));
-      std::array<int, TUNE_N> a;
-      for (int m = 0; m < TUNE_N; m++) a[m] = best[m];
+      std::array<int, TUNE_N + 1> a;
+      for (int m = 0; m <= TUNE_N; m++) a[m] = best[m];
       g_tune_cache[key] = a;
     }
-    apply_tiles(best);
+    apply_tiles(best, best[TUNE_N] != 0);
     if (choice)
       for (int m = 0; m < TUNE_N; m++) choice[m] = best[m];
     if (ms)
