@@ -244,7 +244,11 @@ __device__ __forceinline__ double metric_jac(const Geo& g, int i, int j, int k, 
     double xi, yi, zi, xj, yj, zj, xk, yk, zk;
     bool cross;
     sep_derivs(g, i, j, k, xi, yi, zi, xj, yj, zj, xk, yk, zk, cross);
+#if OCFD_FMA_BUILD
+    if (!cross) return rcp3(xi * yj * zk);
+#else
     if (!cross) return 1.0 / (xi * yj * zk);
+#endif
     double a[9], jac;
     jac_full(xi, yi, zi, xj, yj, zj, xk, yk, zk, a, jac);
     return jac;
@@ -264,7 +268,11 @@ __device__ __forceinline__ void metric_all(const Geo& g, int i, int j, int k, in
     bool cross;
     sep_derivs(g, i, j, k, xi, yi, zi, xj, yj, zj, xk, yk, zk, cross);
     if (!cross) {
+#if OCFD_FMA_BUILD
+      double jac = rcp3(xi * yj * zk);
+#else
       double jac = 1.0 / (xi * yj * zk);
+#endif
       double akx = jac * (yj * zk), aiy = jac * (zk * xi), asz = jac * (xi * yj);
 #pragma unroll
       for (int m = 0; m < 9; m++) { a[m] = 0.0; a1[m] = 0.0; }

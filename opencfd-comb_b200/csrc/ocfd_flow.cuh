@@ -79,6 +79,60 @@ __device__ __forceinline__ void split_point(double Et1, double p1, double c1, do
   }
 }
 
+#if OCFD_FMA_BUILD
+// Steger-Warming along one grid direction of a diagonal metric (A along velocity component DIR):
+// split_point with ss = |A|, (gamma - 1) = p / Et and W2 = (3 - gamma) gamma Et / (2 d), which leaves
+// three reciprocals and one square root of its four divisions and two square roots, and the zeros of
+// the metric vector out of the products. The split of the C + 8 points per C cells is half of a
+// HYBRID sweep's operations and a third of a WENO5 sweep's. ms per step of the x / y / z flow sweeps:
+// 1024x160x32 HYBRID 1.87 / 2.02 / 2.55 -> 1.65 / 1.87 / 2.19, 64^3 WENO5 0.173 / 0.172 / 0.178 ->
+// 0.149 / 0.150 / 0.160, 384x256x32 WENO5 1.24 / 1.39 / 1.95 -> 1.14 / 1.28 / 1.95.
+template <int DIR>
+__device__ __forceinline__ void split_sw_diag(double Et, double p, double d, double u, double v, double w, double A,
+                                              double* fp, double* fm) {
+  const double g1 = p * rcp3(Et), gamma = 1.0 + g1, rd = rcp3(d);
+  const double c = sqrt(gamma * p * rd);
+  const double un = DIR == 0 ? u : (DIR == 1 ? v : w);
+  const double ak = A < 0.0 ? -c : c;  // c times the unit normal
+  const double cs = c * fabs(A), E1 = A * un, E2 = E1 - cs, E3 = E1 + cs;
+  const double t0 = 0.5 * d * rcp3(gamma), t1 = 2.0 * g1;
+  const double k0 = 0.5 * (u * u + v * v + w * w), c2 = 0.5 * c * c, cu = ak * un;
+  const double k1 = k0 + c2 - cu, k2 = k0 + c2 + cu;  // kinetic energies at un -+ c
+  const double W2 = 0.5 * (2.0 - g1) * gamma * Et * rd;
+  const double P1 = t0 * t1 * 0.5 * (E1 + fabs(E1)), P2 = t0 * 0.5 * (E2 + fabs(E2)), P3 = t0 * 0.5 * (E3 + fabs(E3));
+  const double M1 = t0 * t1 * E1 - P1, M2 = t0 * E2 - P2, M3 = t0 * E3 - P3;
+  auto comp = [&](double e1, double e2, double e3, double* f) {
+    const double m = e1 + e2 + e3, a = (e3 - e2) * ak;
+    f[0] = m;
+    f[1] = m * u + (DIR == 0 ? a : 0.0);
+    f[2] = m * v + (DIR == 1 ? a : 0.0);
+    f[3] = m * w + (DIR == 2 ? a : 0.0);
+    f[4] = e1 * k0 + e2 * k1 + e3 * k2 + W2 * (e2 + e3);
+  };
+  comp(P1, P2, P3, fp);
+  comp(M1, M2, M3, fm);
+}
+// Lax-Friedrichs along one grid direction of a diagonal metric
+template <int DIR>
+__device__ __forceinline__ void split_llf_diag(double Et, double p, double d, double u, double v, double w, double A,
+                                               double* fp, double* fm) {
+  const double c = sqrt(fma(p, rcp3(Et), 1.0) * p * rcp3(d));
+  const double un = A * (DIR == 0 ? u : (DIR == 1 ? v : w)), lam = fabs(un) + fabs(A) * c;
+  const double E0 = Et + 0.5 * d * (u * u + v * v + w * w);
+  const double a = 0.5 * (un + lam), b = 0.5 * (un - lam), hp = 0.5 * A * p;
+  fp[0] = d * a;
+  fp[1] = fp[0] * u + (DIR == 0 ? hp : 0.0);
+  fp[2] = fp[0] * v + (DIR == 1 ? hp : 0.0);
+  fp[3] = fp[0] * w + (DIR == 2 ? hp : 0.0);
+  fp[4] = E0 * a + 0.5 * p * un;
+  fm[0] = d * b;
+  fm[1] = fm[0] * u + (DIR == 0 ? hp : 0.0);
+  fm[2] = fm[0] * v + (DIR == 1 ? hp : 0.0);
+  fm[3] = fm[0] * w + (DIR == 2 ? hp : 0.0);
+  fm[4] = E0 * b + 0.5 * p * un;
+}
+#endif
+
 // Tile shapes: C cells along the sweep x NL pencils. x sweeps run along the contiguous index, so
 // a tile is a long chunk of few lines; y / z sweeps put NL contiguous i-lines side by side and a
 // chunk along j / k. Every shape makes the split phase (C + 8 points of NL pencils) a whole
@@ -191,6 +245,27 @@ __global__ void __launch_bounds__(FLUX_THREADS, SCALAR ? OCFD_SCALAR_FLUX_MINB :
     if (threadIdx.x == 0) *sqn = 0;
     __syncthreads();
   }
+#if OCFD_FMA_BUILD
+  // On a tensor-product grid the metric vector lies along the sweep everywhere but the non-periodic
+  // end planes (and halos), and its one component does not change along a y / z line, which a thread
+  // stays on (256 is a multiple of NL): formed once. Along x the plane's factor is. (In the species
+  // sweeps, whose 64 registers are full, the second path costs more than it saves: 7.95 against 8.2 ms
+  // per step on the 384x256x32 jet.)
+  bool line_diag = false;
+  double A0 = 0.0;
+  auto in_core = [&](int dir, int ii, int nn) { return cC.iper[dir] || (ii > 1 && ii < nn); };
+  static_assert(DIR == 0 || FLUX_THREADS % NL == 0, "a thread stays on one line");
+  if constexpr (SEP && !SCALAR) {
+    if (DIR == 0) {
+      line_diag = in_core(2, bz, cC.nz);
+      A0 = a.g.d1[2][bz + OCFD_L - 1];
+    } else {
+      const int il = l0 + (int)threadIdx.x % NL;
+      line_diag = il <= nl_max && in_core(0, il, cC.nx) && (DIR == 1 ? in_core(2, bz, cC.nz) : in_core(1, bz, cC.ny));
+      if (line_diag) A0 = a.g.d1[0][il + OCFD_L - 1] * a.g.d1[DIR == 1 ? 2 : 1][bz + OCFD_L - 1];
+    }
+  }
+#endif
 
   // phase 1 (uniform trip count: the warp-wide ballot below needs every lane)
   for (int base = 0; base < P * NL; base += FLUX_THREADS) {
@@ -205,9 +280,20 @@ __global__ void __launch_bounds__(FLUX_THREADS, SCALAR ? OCFD_SCALAR_FLUX_MINB :
       int i, j, k;
       coords(s, l, i, j, k);
       const int q = hidx(i, j, k);
-      double A1, A2, A3;
-      metric_dir<SEP>(a.g, DIR, i, j, k, q, A1, A2, A3);
+      bool diag = false;
+#if OCFD_FMA_BUILD
+      double Ad = A0;
+      if constexpr (SEP && !SCALAR) {
+        diag = line_diag && in_core(DIR, s, n);
+        if (DIR == 0) {
+          diag = diag && in_core(1, j, cC.ny);
+          Ad = A0 * a.g.d1[1][j + OCFD_L - 1];
+        }
+      }
+#endif
       if constexpr (SCALAR) {
+        double A1, A2, A3;
+        metric_dir<SEP>(a.g, DIR, i, j, k, q, A1, A2, A3);
         double vs = A1 * __ldg(a.u + q) + A2 * __ldg(a.v + q) + A3 * __ldg(a.w + q);
 #pragma unroll
         for (int c = 0; c < NC; c++) {
@@ -217,9 +303,20 @@ __global__ void __launch_bounds__(FLUX_THREADS, SCALAR ? OCFD_SCALAR_FLUX_MINB :
         }
       } else {
         double pp = __ldg(a.p + q), et = __ldg(a.Et + q), dd = __ldg(a.d + q);
-        double gamma = pp / et + 1.0;
-        double cc = sqrt(gamma * pp / dd);  // comput_cc
-        split_point<SPLIT>(et, pp, cc, dd, __ldg(a.u + q), __ldg(a.v + q), __ldg(a.w + q), A1, A2, A3, fp, fm);
+#if OCFD_FMA_BUILD
+        if (diag) {
+          const double uu = __ldg(a.u + q), vv = __ldg(a.v + q), ww = __ldg(a.w + q);
+          if (SPLIT == OCFD_SPLIT_SW) split_sw_diag<DIR>(et, pp, dd, uu, vv, ww, Ad, fp, fm);
+          else split_llf_diag<DIR>(et, pp, dd, uu, vv, ww, Ad, fp, fm);
+        }
+#endif
+        if (!diag) {
+          double A1, A2, A3;
+          metric_dir<SEP>(a.g, DIR, i, j, k, q, A1, A2, A3);
+          double gamma = pp / et + 1.0;
+          double cc = sqrt(gamma * pp / dd);  // comput_cc
+          split_point<SPLIT>(et, pp, cc, dd, __ldg(a.u + q), __ldg(a.v + q), __ldg(a.w + q), A1, A2, A3, fp, fm);
+        }
       }
     } else {
 #pragma unroll
@@ -434,7 +531,13 @@ __global__ void __launch_bounds__(FLUX_THREADS, SCALAR ? OCFD_SCALAR_FLUX_MINB :
     coords(s0 + t, l, i, j, k);
     const int nn = nidx(i, j, k);
     double ajac = 0.0;
-    if (DIR == 2) ajac = metric_jac<SEP>(a.g, i, j, k, hidx(i, j, k));
+    if (DIR == 2) {
+#if OCFD_FMA_BUILD
+      if (SEP && line_diag && in_core(2, k, n)) ajac = rcp3(A0 * a.g.d1[2][k + OCFD_L - 1]);
+      else
+#endif
+        ajac = metric_jac<SEP>(a.g, i, j, k, hidx(i, j, k));
+    }
     const int i0 = iidx(t, l), i1 = iidx(t + 1, l);
 #pragma unroll
     for (int c = 0; c < NC; c++) {
