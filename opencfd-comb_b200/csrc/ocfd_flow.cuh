@@ -1384,28 +1384,29 @@ __global__ void __launch_bounds__(32 * NS, OCFD_TRANSPORT_MINB) k_transport(cons
 // wrap around; a non-periodic face halo is left untouched (MPI_PROC_NULL).
 struct ExchArgs {
   double* f[24];
+  unsigned char mask[24];  // which directions to exchange each field along (bit d)
   int nf;
-  int dirmask;  // which directions to exchange (bit d)
 };
 static __global__ void k_exchange(ExchArgs a) {
   // thread grid: x = face point, y = field
   const int fidx = blockIdx.y;
   if (fidx >= a.nf) return;
   double* f = a.f[fidx];
+  const int mask = a.mask[fidx];
   const int L = OCFD_L;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nxz = L * cC.ny * cC.nz, nyz = L * cC.nx * cC.nz, nzz = L * cC.nx * cC.ny;
-  if ((a.dirmask & 1) && cC.iper[0] && t < nxz) {
+  if ((mask & 1) && cC.iper[0] && t < nxz) {
     int l = t % L, j = (t / L) % cC.ny + 1, k = t / L / cC.ny + 1;
     f[hidx(cC.nx + 1 + l, j, k)] = f[hidx(1 + l, j, k)];
     f[hidx(1 - L + l, j, k)] = f[hidx(cC.nx + 1 - L + l, j, k)];
   }
-  if ((a.dirmask & 2) && cC.iper[1] && t < nyz) {
+  if ((mask & 2) && cC.iper[1] && t < nyz) {
     int i = t % cC.nx + 1, l = (t / cC.nx) % L, k = t / cC.nx / L + 1;
     f[hidx(i, cC.ny + 1 + l, k)] = f[hidx(i, 1 + l, k)];
     f[hidx(i, 1 - L + l, k)] = f[hidx(i, cC.ny + 1 - L + l, k)];
   }
-  if ((a.dirmask & 4) && cC.iper[2] && t < nzz) {
+  if ((mask & 4) && cC.iper[2] && t < nzz) {
     int i = t % cC.nx + 1, j = (t / cC.nx) % cC.ny + 1, l = t / cC.nx / cC.ny;
     f[hidx(i, j, cC.nz + 1 + l)] = f[hidx(i, j, 1 + l)];
     f[hidx(i, j, 1 - L + l)] = f[hidx(i, j, cC.nz + 1 - L + l)];
@@ -1764,25 +1765,27 @@ __device__ __forceinline__ void face_apply(const BcArgs& a, int i, int j, int k,
   a.f[3 * N + nn] = dd * ww;
   a.f[4 * N + nn] = et + dd * (uu * uu + vv * vv + ww * ww) * 0.5;
 }
+// one thread per face cell: the x faces, the y faces without their x edges, the z faces without edges
 template <int NS>
-__global__ void k_bc_faces(BcArgs a, int group) {
+__global__ void k_bc_faces(BcArgs a) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nx = cC.nx, ny = cC.ny, nz = cC.nz;
+  const int n0 = 2 * ny * nz, n1 = 2 * (nx - 2) * nz, n2 = 2 * (nx - 2) * (ny - 2);
   int i, j, k;
-  if (group == 0) {
-    if (t >= 2 * ny * nz) return;
+  if (t < n0) {
     i = (t & 1) ? nx : 1;
     int r = t >> 1;
     j = r % ny + 1;
     k = r / ny + 1;
-  } else if (group == 1) {
-    if (t >= 2 * (nx - 2) * nz) return;
+  } else if (t < n0 + n1) {
+    t -= n0;
     j = (t & 1) ? ny : 1;
     int r = t >> 1;
     i = r % (nx - 2) + 2;
     k = r / (nx - 2) + 1;
   } else {
-    if (t >= 2 * (nx - 2) * (ny - 2)) return;
+    t -= n0 + n1;
+    if (t >= n2) return;
     k = (t & 1) ? nz : 1;
     int r = t >> 1;
     i = r % (nx - 2) + 2;

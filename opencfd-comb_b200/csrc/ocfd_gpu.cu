@@ -206,34 +206,35 @@ void prof_collect() {
 
 inline unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
-void exchange(std::initializer_list<double*> fields, int dirmask) {
-  ExchArgs a{};
-  a.nf = 0;
-  for (double* f : fields) a.f[a.nf++] = f;
-  a.dirmask = dirmask;
-  bool any = false;
-  for (int dd = 0; dd < 3; dd++)
-    if ((dirmask >> dd & 1) && L->P.iperiodic[dd]) any = true;
-  if (!any || a.nf == 0) return;
+// periodic wrap of up to 24 fields per launch, each along the directions of its mask; fields without
+// a periodic direction in their mask need none
+void exchange_masks(const std::vector<std::pair<double*, int>>& fields) {
+  int per = 0;
+  for (int dd = 0; dd < 3; dd++) per |= L->P.iperiodic[dd] ? 1 << dd : 0;
   const int nx = L->P.nx, ny = L->P.ny, nz = L->P.nz;
-  long long mx = std::max((long long)ny * nz, std::max((long long)nx * nz, (long long)nx * ny)) * OCFD_L;
-  KTimer t(KC_EXCH);
-  k_exchange<<<dim3(nblk(mx, 256), a.nf), 256, 0, L->st>>>(a);
-  LAUNCH_CHECK();
-}
-void exchange_v(const std::vector<double*>& fields, int dirmask) {
-  for (size_t s = 0; s < fields.size(); s += 24) {
-    ExchArgs a{};
-    a.nf = 0;
-    for (size_t m = s; m < fields.size() && m < s + 24; m++) a.f[a.nf++] = fields[m];
-    a.dirmask = dirmask;
-    const int nx = L->P.nx, ny = L->P.ny, nz = L->P.nz;
-    long long mx = std::max((long long)ny * nz, std::max((long long)nx * nz, (long long)nx * ny)) * OCFD_L;
+  const long long mx = std::max((long long)ny * nz, std::max((long long)nx * nz, (long long)nx * ny)) * OCFD_L;
+  ExchArgs a{};
+  auto flush = [&]() {
+    if (a.nf == 0) return;
     KTimer t(KC_EXCH);
     k_exchange<<<dim3(nblk(mx, 256), a.nf), 256, 0, L->st>>>(a);
     LAUNCH_CHECK();
+    a.nf = 0;
+  };
+  for (const auto& f : fields) {
+    if (!(f.second & per)) continue;
+    a.f[a.nf] = f.first;
+    a.mask[a.nf++] = (unsigned char)(f.second & per);
+    if (a.nf == 24) flush();
   }
+  flush();
 }
+void exchange_v(const std::vector<double*>& fields, int dirmask) {
+  std::vector<std::pair<double*, int>> v;
+  for (double* f : fields) v.push_back({f, dirmask});
+  exchange_masks(v);
+}
+void exchange(std::initializer_list<double*> fields, int dirmask) { exchange_v(std::vector<double*>(fields), dirmask); }
 
 // ---- flux dispatch (kernels compiled in ocfd_flux_{x,y,z}.cu) ----
 // group = 0: the flow fluxes; else a scalar sweep of every species, group species per block
@@ -327,11 +328,7 @@ void ocfd_bc_t() {
   }
   {
     KTimer t(KC_BC);
-    k_bc_faces<NS><<<nblk(2LL * ny * nz, 128), 128, 0, L->st>>>(a, 0);
-    LAUNCH_CHECK();
-    k_bc_faces<NS><<<nblk(2LL * (nx - 2) * nz, 128), 128, 0, L->st>>>(a, 1);
-    LAUNCH_CHECK();
-    k_bc_faces<NS><<<nblk(2LL * (nx - 2) * (ny - 2), 128), 128, 0, L->st>>>(a, 2);
+    k_bc_faces<NS><<<nblk(2LL * ny * nz + 2LL * (nx - 2) * nz + 2LL * (nx - 2) * (ny - 2), 128), 128, 0, L->st>>>(a);
     LAUNCH_CHECK();
   }
   for (int face = 0; face < 6; face++) {
@@ -483,9 +480,9 @@ void flow_rhs_t(const FluxArgs& fa) {
       KTimer t(KC_VISC_EV);
       visc_ev_launch<NS>(visc_args<NS>());
     }
-    exchange({L->ev[0], L->ev[1], L->ev[2], L->ev[3]}, 1);
-    exchange({L->ev[4], L->ev[5], L->ev[6], L->ev[7]}, 2);
-    exchange({L->ev[8], L->ev[9], L->ev[10], L->ev[11]}, 4);
+    std::vector<std::pair<double*, int>> fl;  // Ev1, Ev2, Ev3 along x, y, z
+    for (int m = 0; m < 12; m++) fl.push_back({L->ev[m], 1 << (m / 4)});
+    exchange_masks(fl);
   };
   // k_visc_ev reads only the primitives (and, for N_SPEC > 1, the transport and enthalpy fluxes
   // computed above) and writes only Ev, while the flux sweeps write du: the two run side by side
@@ -650,11 +647,10 @@ void stage_rhs_t(int krk, double dt1, bool rk) {
         if (nb > 0) L->sep ? ev(k_scal_ev<NS, true>) : ev(k_scal_ev<NS, false>);
         LAUNCH_CHECK();
       }
-      for (int dd = 0; dd < 3; dd++) {
-        std::vector<double*> fl;
-        for (int m = 0; m < NS; m++) fl.push_back(L->se[dd] + (size_t)m * H);
-        exchange_v(fl, 1 << dd);
-      }
+      std::vector<std::pair<double*, int>> fl;
+      for (int dd = 0; dd < 3; dd++)
+        for (int m = 0; m < NS; m++) fl.push_back({L->se[dd] + (size_t)m * H, 1 << dd});
+      exchange_masks(fl);
     }
     if (spfork) {
       CK(cudaEventRecord(L->ev_se_done, L->st));
