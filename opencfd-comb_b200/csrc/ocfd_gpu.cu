@@ -61,8 +61,9 @@ struct CudaError : std::runtime_error {
 #define LAUNCH_CHECK() CK(cudaGetLastError())
 
 // kernel classes for event timing
-// (species work of N_SPEC > 1, by kernel family: transport = k_transport, species_flux = the
-// scalar k_flux sweeps, species_visc = k_ci + k_scal_ev + k_scal_div, species_rk = k_scal_rk)
+// (species work of N_SPEC > 1, by kernel family: transport = k_transport(_fit), species_flux = the
+// scalar k_flux sweeps, species_visc = k_ci + k_spec_ev + k_spec_div and the face cells' k_scal_ev +
+// k_scal_div, species_rk = k_scal_rk)
 enum KClass { KC_FLUX_X = 0, KC_FLUX_Y, KC_FLUX_Z, KC_VISC_EV, KC_VISC_DIV, KC_RK_PRIMS, KC_EXCH, KC_BC, KC_SENSOR,
               KC_TRANSPORT, KC_SPECIES_FLUX, KC_SPECIES_VISC, KC_SPECIES_RK, KC_CHEM, KC_OTHER, KC_NUM };
 const char* kc_names[KC_NUM] = {"flux_x", "flux_y", "flux_z", "visc_ev", "visc_div", "rk_prims", "exchange",
@@ -145,6 +146,8 @@ struct Lib {
   double *b_di = nullptr, *b_e = nullptr, *b_dt = nullptr;
   int *b_nsub = nullptr, *b_perm = nullptr, *b_hist = nullptr, *b_counter = nullptr, *b_nfail = nullptr;
   size_t b_cap = 0;
+  char* b_stage = nullptr;  // device copies of a host batch (ocfd_gpu_chem_batch), grown on demand
+  size_t b_stage_bytes = 0;
   int b_last[2] = {0, 0};  // the last batch call's Newton non-convergences and bad reactors
   // profiling
   bool prof = false;
@@ -1176,6 +1179,7 @@ void release() {
   if (L->shost) cudaFreeHost(L->shost);
   if (L->ht_host) cudaFreeHost(L->ht_host);
   if (L->b_di) cudaFree(L->b_di);
+  if (L->b_stage) cudaFree(L->b_stage);
   if (L->ht_seq) cudaFree(L->ht_seq);
   if (L->ht_seq_host) cudaFreeHost(L->ht_seq_host);
   for (auto& e : L->uev)
@@ -2278,12 +2282,23 @@ int ocfd_gpu_chem_batch(int n, double* di, double* e, const double* dt, const in
     L->b_last[0] = L->b_last[1] = 0;
     if (n == 0) return 0;
     const int NS = L->NS;
-    double *ddi, *de, *ddt;
-    int* dns = nullptr;
-    CK(cudaMallocAsync(&ddi, sizeof(double) * (size_t)n * NS, L->st));
-    CK(cudaMallocAsync(&de, sizeof(double) * n, L->st));
-    CK(cudaMallocAsync(&ddt, sizeof(double) * n, L->st));
-    if (nsub) CK(cudaMallocAsync(&dns, sizeof(int) * n, L->st));
+    // kept between calls up to STAGE_KEEP (a small batch's time was in allocating and freeing four
+    // arrays), given back with the set-up
+    constexpr size_t STAGE_KEEP = (size_t)64 << 20;
+    auto drop = [&]() {
+      if (L->b_stage) CK(cudaFree(L->b_stage));
+      L->b_stage = nullptr;
+      L->b_stage_bytes = 0;
+    };
+    const size_t need = sizeof(double) * (size_t)n * (NS + 2) + sizeof(int) * (size_t)n;
+    if (need > L->b_stage_bytes) {
+      drop();
+      CK(cudaMalloc(&L->b_stage, need));
+      L->b_stage_bytes = need;
+    }
+    double* ddi = reinterpret_cast<double*>(L->b_stage);
+    double *de = ddi + (size_t)n * NS, *ddt = de + n;
+    int* dns = nsub ? reinterpret_cast<int*>(ddt + n) : nullptr;
     CK(cudaMemcpyAsync(ddi, di, sizeof(double) * (size_t)n * NS, cudaMemcpyHostToDevice, L->st));
     CK(cudaMemcpyAsync(de, e, sizeof(double) * n, cudaMemcpyHostToDevice, L->st));
     CK(cudaMemcpyAsync(ddt, dt, sizeof(double) * n, cudaMemcpyHostToDevice, L->st));
@@ -2292,11 +2307,8 @@ int ocfd_gpu_chem_batch(int n, double* di, double* e, const double* dt, const in
     if (rc != 0 && rc != OCFD_ERR_CHEM) return rc;
     CK(cudaMemcpyAsync(di, ddi, sizeof(double) * (size_t)n * NS, cudaMemcpyDeviceToHost, L->st));
     CK(cudaMemcpyAsync(e, de, sizeof(double) * n, cudaMemcpyDeviceToHost, L->st));
-    CK(cudaFreeAsync(ddi, L->st));
-    CK(cudaFreeAsync(de, L->st));
-    CK(cudaFreeAsync(ddt, L->st));
-    if (dns) CK(cudaFreeAsync(dns, L->st));
     CK(cudaStreamSynchronize(L->st));
+    if (L->b_stage_bytes > STAGE_KEEP) drop();
     if (rc) g_err = "chemistry: " + std::to_string(L->b_last[1]) +
                     " reactor(s) with a zero Gauss pivot or a non-finite result (their values are returned as computed)";
     return rc;
