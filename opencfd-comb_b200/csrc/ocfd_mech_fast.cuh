@@ -11,7 +11,7 @@
 //    N2 drops out, and the elimination is unpivoted in registers. A lane whose elimination met a
 //    multiplier above MULT_MAX (or whose state the forms above do not cover: T below T_MIN or above
 //    the fits) repeats the sub-step with the pivoted general step.
-// Bound by FP64 issue and its latency at eight warps per SM (208 registers, most of them the 8 x 8
+// Bound by FP64 issue and its latency at eight warps per SM (255 registers, half of them the 8 x 8
 // matrix; the rates of progress wait in shared memory until it is assembled, so the two phases'
 // values are not live together). About 1500 FP64 operations per sub-step against some 3500 with the
 // matrix in shared memory, 42 equilibrium and rate exponentials of 20, and a division per pivot row.
