@@ -572,7 +572,7 @@ void stage_rhs_t(int krk, double dt1, bool rk) {
   // the reference's species loop; Dus of species m is dus + m N). The species sweeps read only di
   // and the velocities and write only Dus, and nothing of the flow part reads di, so the sweeps,
   // the species divergence (after the species viscous fluxes) and the species RK update run on a
-  // third stream beside k_ci / k_scal_ev and the flow part (branches of the step's graph), joined
+  // third stream beside k_ci / k_spec_ev and the flow part (branches of the step's graph), joined
   // before k_rk_prims, which reads the updated di. Each kernel writes what it wrote before, so the
   // results do not depend on the overlap. The per-kernel timing mode keeps everything in order.
   const bool spfork = NS > 1 && L->fork_species && !L->prof && L->st3;
