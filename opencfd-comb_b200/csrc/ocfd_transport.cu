@@ -92,9 +92,15 @@ __global__ void __launch_bounds__(OCFD_TFIT_THREADS, OCFD_TFIT_MINB)
     X[m] = di[(size_t)m * cC.H + q] * cF.rMi[m];
     X0 += X[m];
   }
-  X0 = rcp3(X0);
+  // mole fractions: the product with 1 / X0 and its remainder, so that a cell of one species alone gets
+  // X = 1 exactly, as the division gives it. Its 1 - X is then 0; one unit in the last place of X
+  // instead would be divided by ds = 1e-20 below.
+  const double rX = rcp3(X0);
 #pragma unroll
-  for (int m = 0; m < NS; m++) X[m] *= X0;
+  for (int m = 0; m < NS; m++) {
+    const double x = X[m] * rX;
+    X[m] = fma(fma(-x, X0, X[m]), rX, x);
+  }
   // diffusion: ds_k = sum over j != k of X_j / D_kj, every pair's exponential once
   double ds[NS];
 #pragma unroll

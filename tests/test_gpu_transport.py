@@ -52,3 +52,27 @@ def test_transport_fit_against_oracle(oracle, ns, n):
         for m in range(len(r)):
             want, got = r[m] - s[m], a[m] - b[m]
             assert np.abs(got - want).max() <= 1e-13 * np.abs(r[m]).max() + 1e-10 * np.abs(want).max(), m
+
+
+def unmixed(ns, n=12):
+    """two of the species side by side, each alone in its half of a periodic box"""
+    c = case(n, ns, ns)
+    half = np.where(np.arange(n) < n // 2, 1.0, 0.0)
+    d = c.di.sum(axis=0)
+    c.di = np.zeros_like(c.di)
+    c.di[0], c.di[1] = d * half, d * (1.0 - half)
+    return c
+
+
+@pytest.mark.parametrize("ns", [2, 9])
+def test_cells_of_one_species(oracle, ns):
+    """X = 1 exactly where a species is alone: its diffusion coefficient (1 - X) / (sum + 1e-20) is 0
+    there. Last-place changes of the initial state move the oracle's own increments by less than a
+    hundredth of the bound."""
+    c = unmixed(ns)
+    gv, gi = steps(solver.Solver, c)
+    ov, oi = steps(oracle.OracleSolver, c)
+    for a, b, r, s in ((gv[0], gi[0], ov[0], oi[0]), (gv[1], gi[1], ov[1], oi[1])):
+        for m in range(len(r)):
+            want, got = r[m] - s[m], a[m] - b[m]
+            assert np.abs(got - want).max() <= 1e-13 * np.abs(r[m]).max() + 1e-10 * np.abs(want).max(), m
