@@ -2149,6 +2149,9 @@ int ocfd_gpu_chem_setup(const ocfd_thermo* th, const ocfd_kinetics* kin, int rea
     L->hc.ns = th->n_spec;
     L->hc.const_p = 0;  // the reference's constant-volume reactor unless ocfd_gpu_chem_constant_pressure(1)
     CK(mech_setup(L->hc));
+    // an open flow solver reads the new thermodynamics too
+    CK(species_setup(L->hc, L->NS));
+    CK(transport_fit_masses(L->hc, L->NS));
     L->have_kin = true;
     CK(cudaMemcpyToSymbol(cC, &L->hc, sizeof(DevConst)));
     return 0;

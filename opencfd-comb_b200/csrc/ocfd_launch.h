@@ -32,6 +32,7 @@ void launch_chem_batch(int ns, int sms, int n, double* di, double* e, const doub
 // fitted mixture transport (Flag_vis = Flag_cond = Flag_diff = 1, N_SPEC 2..9; ocfd_transport.cu);
 // the set-up fills its constants and is not for stream capture
 cudaError_t transport_fit_setup(const DevConst& c, int ns);
+cudaError_t transport_fit_masses(const DevConst& c, int ns);  // the molar masses alone, after ocfd_gpu_chem_setup
 void launch_transport_fit(int ns, long long N, const double* T, const double* p, const double* di, double* amu,
                           double* amk, double* amd, cudaStream_t st);
 // species viscous terms on tensor-product grids (ocfd_species.cu); krk = 1..3 runs the species RK

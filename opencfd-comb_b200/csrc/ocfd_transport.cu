@@ -4,6 +4,7 @@
 // comput_diffusion_coeff of TRANSPORT_modules.f90:259-426). Other flag combinations keep
 // k_transport (ocfd_flow.cuh).
 #include <cmath>
+#include <cstddef>
 #include <stdexcept>
 
 #include "ocfd_device.cuh"
@@ -50,6 +51,15 @@ cudaError_t transport_fit_setup(const DevConst& c, int ns) {
   }
   const cudaError_t e = cudaMemcpyToSymbol(cF, &t, sizeof(t));
   return e != cudaSuccess ? e : exp2_tab_setup();
+}
+
+// ocfd_gpu_chem_setup on an open flow solver replaces the masses of the mole fractions; the fits and the
+// pair constants stay those of ocfd_gpu_init, as in k_transport.
+cudaError_t transport_fit_masses(const DevConst& c, int ns) {
+  if (ns < 2 || ns > TF_NS) return cudaSuccess;
+  double r[TF_NS] = {};
+  for (int k = 0; k < ns; k++) r[k] = 1.0 / c.Mi[k];
+  return cudaMemcpyToSymbol(cF, r, sizeof(r), offsetof(TransFit, rMi));
 }
 
 // ---------------------------------------------------------------- arithmetic
