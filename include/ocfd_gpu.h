@@ -296,7 +296,8 @@ int ocfd_gpu_ana_average(int upload, double* fields, int* k_average, double* t_a
 
 /* Stencil tile autotuner (no counterpart in the reference, whose loops have no tiles). A tile
  * choice is int[9] = {flux tile shape of the x, y, z flow sweeps (0, 1, 2); k planes per block of
- * the viscous-flux kernel and of its divergence kernel; metric form of the flux sweeps, the
+ * the viscous-flux kernel and of its divergence kernel (0 for the latter: both kernels with one thread
+ * per cell, the former's planes without effect); metric form of the flux sweeps, the
  * viscous-flux kernel and the divergence kernel (0 computed from the 1-D grid derivatives of a
  * tensor-product grid, 1 read from the 19 stored arrays, which are then computed once; a general
  * grid always reads them); stream switches, bit 0: the viscous-flux kernel runs beside the flux
@@ -314,10 +315,9 @@ int ocfd_gpu_ana_average(int upload, double* fields, int* k_average, double* t_a
  * best tiles: flux x, y, z, k_visc_ev, k_visc_div, then the flow right-hand side of a stage with
  * the viscous flux after and beside the flux sweeps, then a stage's right-hand sides without the
  * species RK update with the species chain in order and on the third stream (-1 where not timed).
- * The launches write only scratch arrays, so the solution is unchanged. Default choice
- * {0, 0, 0, 16, 16, 0, 0, 0, 3}, with the two viscous kernels in their per-cell forms until a choice
- * is set or tuned; the tuner also times the per-cell k_visc_ev (not among the 27 times) and keeps it
- * where it is the fastest. */
+ * The launches write only scratch arrays, so the solution is unchanged. The tuner also times the
+ * per-cell k_visc_ev (not among the 27 times) and takes the per-cell pair of viscous kernels or the
+ * marching pair, whichever is faster together. Default choice {0, 0, 0, 16, 0, 0, 0, 0, 3}. */
 int ocfd_gpu_autotune(int reps, int* choice, double* ms);
 int ocfd_gpu_set_tiles(const int* choice);
 int ocfd_gpu_get_tiles(int* choice);

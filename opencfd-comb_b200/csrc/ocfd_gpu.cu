@@ -115,10 +115,8 @@ struct Lib {
   // stencil tile choices (ocfd_gpu_set_tiles / ocfd_gpu_autotune): flow-flux tile shape per
   // sweep direction, k planes per block of k_visc_ev and k_visc_div
   int flux_ts[3] = {0, 0, 0};
-  int kc_ev = VE_KC, kc_div = VE_KC;
-  // the per-cell forms of the two viscous kernels instead of the marching ones: until a choice is
-  // set or tuned, and (k_visc_ev) when the tuner found it faster than every k chunk
-  bool ev_pc = true, div_pc = true;
+  // (kc_div = 0: both in their per-cell forms, kc_ev without effect)
+  int kc_ev = VE_KC, kc_div = 0;
   // metric form per kernel family on a tensor-product grid: false = computed from the 1-D
   // derivatives (separable), true = read from the 19 stored arrays (allocated on first use)
   bool met_flux = false, met_ev = false, met_div = false;
@@ -448,7 +446,7 @@ ViscArgs visc_args() {
   for (int dd = 0; dd < 3; dd++)
     for (int m = 0; m < 4; m++) va.ev[dd][m] = L->ev[4 * dd + m];
   va.g = L->geo;
-  va.kc = L->ev_pc ? 0 : L->kc_ev;
+  va.kc = L->kc_div == 0 ? 0 : L->kc_ev;
   return va;
 }
 DivArgs div_args() {
@@ -456,7 +454,7 @@ DivArgs div_args() {
   for (int m = 0; m < 12; m++) da.ev[m] = L->ev[m];
   da.du = L->du;
   da.g = L->geo;
-  da.kc = L->div_pc ? 0 : L->kc_div;
+  da.kc = L->kc_div;
   return da;
 }
 template <int NS>
@@ -705,14 +703,14 @@ void chem_t(double dt2, int nsub) {
 }
 
 // ---------------------------------------------------------------- stencil tile autotuner
-// Tile choices {flux x, y, z shape; k_visc_ev, k_visc_div k planes per block; metric form of the
-// flux sweeps, k_visc_ev, k_visc_div; k_visc_ev beside the flux sweeps on a second stream or after
-// them}. Every choice gives bit-identical results (a tile decides
+// Tile choices {flux x, y, z shape; k_visc_ev, k_visc_div k planes per block (0 for k_visc_div: both
+// kernels in their per-cell forms); metric form of the flux sweeps, k_visc_ev, k_visc_div; k_visc_ev
+// beside the flux sweeps on a second stream or after them}. Every choice gives bit-identical results (a tile decides
 // which block computes a point, not how; the stored metric arrays hold the values the separable
 // form computes), so the tuner is free to pick by time alone. Choices are remembered per
 // configuration in the process.
 constexpr int TUNE_N = 9, TUNE_TIMES = 3 * FLUX_TILE_SHAPES + 9 + 5 + 2 + 2;
-std::map<std::string, std::array<int, TUNE_N + 1>> g_tune_cache;  // the choice and best[TUNE_N]
+std::map<std::string, std::array<int, TUNE_N>> g_tune_cache;
 
 std::string tune_key() {
   const ocfd_params& P = L->P;
@@ -754,12 +752,10 @@ void ensure_stored_metrics() {
   set_geo_device_ptrs();
 }
 
-void apply_tiles(const int* c, bool ev_pc = false) {
+void apply_tiles(const int* c) {
   for (int d = 0; d < 3; d++) L->flux_ts[d] = c[d];
   L->kc_ev = c[3];
   L->kc_div = c[4];
-  L->ev_pc = ev_pc;
-  L->div_pc = false;  // c[4] = 0 names the per-cell form
   if (L->sep && (c[5] | c[6] | c[7])) ensure_stored_metrics();
   L->met_flux = c[5] != 0;
   L->met_ev = c[6] != 0;
@@ -773,7 +769,7 @@ void apply_tiles(const int* c, bool ev_pc = false) {
 // launches between two events) and applies the fastest; the launches write only scratch arrays
 // (du, Ev, the hybrid sensor) that every stage recomputes before it reads them
 template <int NS>
-void tune_t(int reps, int* best, double* ms) {  // best[TUNE_N]: k_visc_ev's per-cell form wins
+void tune_t(int reps, int* best, double* ms) {
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -807,37 +803,34 @@ void tune_t(int reps, int* best, double* ms) {  // best[TUNE_N]: k_visc_ev's per
       }
       L->flux_ts[d] = best[d];
     }
-    best[3] = best[4] = VE_KC;
-    best[TUNE_N] = 0;
-    L->ev_pc = L->div_pc = false;
+    best[3] = VE_KC;
+    best[4] = 0;
     double t_evform = 1e300;  // k_visc_ev in the chosen form
     best[5] = best[6] = best[7] = L->sep ? 0 : 1;
     best[8] = NS > 1 ? 3 : 1;
     for (int m = 3 * FLUX_TILE_SHAPES; m < TUNE_TIMES; m++) ms[m] = -1.0;
     if (P.if_viscous == 1) {
+      // the marching pair, each at its best chunk, or the per-cell pair: whichever is faster together
       double t_ev = 1e300, t_div = 1e300;
+      ViscArgs va = visc_args<NS>();
+      DivArgs da = div_args();
+      int kc_div = VE_KC;
       for (int m = 0; m < 4; m++) {
-        ViscArgs va = visc_args<NS>();
         va.kc = VE_KC_CHOICES[m];
         const double t = timed([&] { visc_ev_launch<NS>(va); });
         ms[3 * FLUX_TILE_SHAPES + m] = t;
         if (t < t_ev) { t_ev = t; best[3] = va.kc; }
       }
-      {
-        ViscArgs va = visc_args<NS>();
-        va.kc = 0;
-        const double t = timed([&] { visc_ev_launch<NS>(va); });
-        best[TUNE_N] = t < t_ev ? 1 : 0;
-        t_evform = std::min(t, t_ev);
-        L->ev_pc = best[TUNE_N] != 0;
-      }
+      va.kc = 0;
+      const double t_evpc = timed([&] { visc_ev_launch<NS>(va); });
       for (int m = 0; m < 5; m++) {  // the four k chunks, then the per-cell form (0)
-        DivArgs da = div_args();
         da.kc = m < 4 ? VE_KC_CHOICES[m] : 0;
         const double t = timed([&] { visc_div_launch(da); });
         ms[3 * FLUX_TILE_SHAPES + 4 + m] = t;
-        if (t < t_div) { t_div = t; best[4] = da.kc; }
+        if (m < 4 && t < t_div) { t_div = t; kc_div = da.kc; }
       }
+      best[4] = t_evpc + ms[3 * FLUX_TILE_SHAPES + 8] <= t_ev + t_div ? 0 : kc_div;
+      t_evform = best[4] == 0 ? t_evpc : t_ev;
     }
     if (L->sep) {  // the stored metric arrays, each family at its best tile
       ensure_stored_metrics();
@@ -859,7 +852,7 @@ void tune_t(int reps, int* best, double* ms) {  // best[TUNE_N]: k_visc_ev's per
       if (P.if_viscous == 1) {
         L->met_ev = true;
         ViscArgs va = visc_args<NS>();
-        va.kc = L->ev_pc ? 0 : best[3];
+        va.kc = best[4] == 0 ? 0 : best[3];
         ms[M0 + 3] = timed([&] { visc_ev_launch<NS>(va); });
         L->met_ev = false;
         best[6] = ms[M0 + 3] < t_evform ? 1 : 0;
@@ -2514,7 +2507,7 @@ int ocfd_gpu_set_tiles(const int* choice) {
       return OCFD_ERR_PARAM;
     }
     if (choice[3] < 1 || choice[4] < 0) {
-      g_err = "k planes per block must be >= 1 (k_visc_div: >= 0, 0 = per-cell form)";
+      g_err = "k planes per block must be >= 1 (k_visc_div: >= 0, 0 = both viscous kernels per cell)";
       return OCFD_ERR_PARAM;
     }
     for (int m = 5; m < 8; m++)
@@ -2547,20 +2540,20 @@ int ocfd_gpu_autotune(int reps, int* choice, double* ms) {
   return guarded([&]() -> int {
     if (!L || !L->flow_ready) { g_err = "state not initialised"; return OCFD_ERR_STATE; }
     if (reps < 0) { g_err = "reps must be >= 0"; return OCFD_ERR_PARAM; }
-    int best[TUNE_N + 1];
+    int best[TUNE_N];
     double t[TUNE_TIMES];
     const std::string key = tune_key();
     auto it = g_tune_cache.find(key);
     if (reps == 0 && it != g_tune_cache.end()) {
-      for (int m = 0; m <= TUNE_N; m++) best[m] = it->second[m];
+      for (int m = 0; m < TUNE_N; m++) best[m] = it->second[m];
       for (int m = 0; m < TUNE_TIMES; m++) t[m] = -1.0;
     } else {
       NS_DISPATCH(L->NS, tune_t<NSV>(reps > 0 ? reps : 3, best, t));
-      std::array<int, TUNE_N + 1> a;
-      for (int m = 0; m <= TUNE_N; m++) a[m] = best[m];
+      std::array<int, TUNE_N> a;
+      for (int m = 0; m < TUNE_N; m++) a[m] = best[m];
       g_tune_cache[key] = a;
     }
-    apply_tiles(best, best[TUNE_N] != 0);
+    apply_tiles(best);
     if (choice)
       for (int m = 0; m < TUNE_N; m++) choice[m] = best[m];
     if (ms)

@@ -102,3 +102,31 @@ def test_bad_tile_choice_is_rejected():
         with pytest.raises(solver.OcfdError):
             g.set_tiles(bad)
     g.close()
+
+
+@pytest.mark.parametrize("tuned", [False, True])
+def test_reported_tiles_are_those_that_run(tuned):
+    """setting what tiles() reports changes nothing: on a 16^3 box the marching viscous-flux kernel takes
+    five times as long as the per-cell one, so another form shows in its time"""
+    c = cases.isotropic(n=16)
+    g = solver.Solver(c)
+    g.init_state()
+    if tuned:
+        g.autotune(reps=3)
+
+    def ms():
+        best = []
+        for _ in range(5):
+            g.profile(True)
+            g.step(c.dt)
+            p = g.profile_read()
+            best.append(p["visc_ev"][0] + p["visc_div"][0])
+        return min(best)
+
+    ms()
+    reported, before = g.tiles(), ms()
+    g.set_tiles(reported)
+    assert g.tiles() == reported
+    assert ms() < 1.8 * before
+    g.profile(False)
+    g.close()
