@@ -110,8 +110,12 @@ __device__ __forceinline__ int nidx(int i, int j, int k) { return (i - 1) + cC.n
 __device__ __forceinline__ unsigned fast_div(unsigned n, unsigned d, unsigned m, int s) {
   return d == 1 ? n : __umulhi(n, m) >> s;
 }
-// 1 / x for normal x: the hardware's approximation (about 2^-23) refined by one third-order Newton
-// (Householder) step, y (1 + e + e^2) with e = 1 - x y; the error e^3 is below the last place
+// 1 / x: the hardware's approximation, of which the high word is given (20 fraction bits), refined by one
+// third-order Newton (Householder) step, y (1 + e + e^2) with e = 1 - x y; the error e^3 <= 2^-60 is below
+// the last place, so the result is within one unit of the quotient for 2^-1022 <= |x| < 2^1022. Above that it
+// is 0; zero, subnormals and infinities give NaN, where a division gives infinity or 0. The callers'
+// arguments are such in states that have already failed (densities, pressures and energies that reached 0 or
+// overflowed), which the step's checks report either way.
 __device__ __forceinline__ double rcp3(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

@@ -22,7 +22,9 @@ static __device__ __forceinline__ void exp2_tab_load(double* tab) {
 // 2^y by table and polynomial (P. T. P. Tang, "Table-driven implementation of the exponential
 // function in IEEE floating-point arithmetic", ACM TOMS 15, 1989): y = n / 64 + r, |r| <= 1 / 128,
 // 2^y = 2^(n >> 6) tab[n & 63] 2^r with the Taylor polynomial of degree 5 (remainder 4e-17). Nine
-// FP64 operations; the binary exponent is added as an integer and saturates at the normal range.
+// FP64 operations, 2.8e-16 for -1022 <= y <= 1022; the binary exponent is added as an integer and saturates
+// there, so that a smaller result than 2^-1022 is about that and not 0 (|y| < 2^25: beyond it the low word
+// wraps). NaN gives NaN, and so do infinities.
 __device__ __forceinline__ double exp2_tab(double y, const double* tab) {
   constexpr double MAGIC = 6755399441055744.0;  // 1.5 2^52: the sum's low word is rint(64 y)
   const double t = fma(y, (double)E2_N, MAGIC);
