@@ -22,9 +22,6 @@ int mech_match(const DevConst& c) {
     }
     if (c.sgm[j] != sg) return MECH_GENERIC;
   }
-#if OCFD_FMA_BUILD
-  if (!mech_fast::usable(c)) return MECH_GENERIC;
-#endif
   return MECH_H2AIR9;
 }
 cudaError_t mech_setup(const DevConst& c) {

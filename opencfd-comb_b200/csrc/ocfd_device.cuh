@@ -18,6 +18,9 @@
 namespace ocfd {
 
 // ---------------------------------------------------------------- constant memory
+// The kernels take up to 9 species (ocfd_gpu_init, ocfd_gpu_chem_setup); the pair tables have that size,
+// since all units' constants share 64 KB.
+constexpr int DEV_SPEC = 9;
 struct DevConst {
   int nx, ny, nz, ns;
   // division of a 31-bit cell index by nx and ny as a multiply-high and a shift (magic numbers of
@@ -58,12 +61,12 @@ struct DevConst {
   int flag_vis, flag_cond, flag_diff;
   double amu0, pr, sc;
   double mu_an[OCFD_MAX_SPEC][4], k_an[OCFD_MAX_SPEC][4];
-  double d_an[OCFD_MAX_SPEC][OCFD_MAX_SPEC][4];
+  double d_an[DEV_SPEC][DEV_SPEC][4];
   // Wilke pair constants of comput_vis_coeff, sqrt(Mi(j)/Mi(k)) and sqrt(8*(1+Mi(k)/Mi(j))):
   // cell-independent, evaluated on the host with the same correctly rounded operations
-  double wk_a[OCFD_MAX_SPEC][OCFD_MAX_SPEC], wk_b[OCFD_MAX_SPEC][OCFD_MAX_SPEC];
+  double wk_a[DEV_SPEC][DEV_SPEC], wk_b[DEV_SPEC][DEV_SPEC];
   // the same pair constants for the multi-species transport kernel: sqrt(wk_a) and 1 / wk_b
-  double wk_c[OCFD_MAX_SPEC][OCFD_MAX_SPEC], wk_binv[OCFD_MAX_SPEC][OCFD_MAX_SPEC];
+  double wk_c[DEV_SPEC][DEV_SPEC], wk_binv[DEV_SPEC][DEV_SPEC];
   // species pairs (a, b), a < b, enumerated a-major: pair p = (pair_a[p], pair_b[p])
   unsigned char pair_a[OCFD_MAX_SPEC * (OCFD_MAX_SPEC - 1) / 2], pair_b[OCFD_MAX_SPEC * (OCFD_MAX_SPEC - 1) / 2];
   unsigned char pair_of[OCFD_MAX_SPEC][OCFD_MAX_SPEC];  // the pair number of (a, b) and (b, a)

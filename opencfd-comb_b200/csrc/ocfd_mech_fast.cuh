@@ -43,7 +43,7 @@ using mech_h2air9::TR_REAC;
 using mech_h2air9::VF;
 using mech_h2air9::VR;
 constexpr int NA = NS - 1;  // reacting species: all but the last (N2)
-constexpr int MAX_RANGES = 3, NRG = MAX_RANGES + 1;  // fit ranges, and the one above the last temperature
+constexpr int NRG = OCFD_NTCT_MAX + 1;  // fit ranges, and the one above the last temperature
 // Below T_MIN the partial products of 2^(F_i) and a rate may leave the exponent range: with the shipped
 // tables they stay within 2^-888 and 2^456 at 90 K, which leaves 2^-134 to the concentrations.
 constexpr double T_MIN = 90.0;
@@ -57,8 +57,9 @@ constexpr bool inert_last() {
 static_assert(inert_last(), "the last species takes part in no reaction");
 
 struct Fast {
-  double e6[NS][NRG][6];  // internal energy of species k per density: R (c0-1), R c1/2, ..., R c4/5, R Ect
-  double g2[NA][NRG][7];  // log2(e) times: c0, -c1/2, -c2/6, -c3/12, -c4/20, c5, -c6
+  // by fit range, so that the range in use is one stretch of the constant cache
+  double e6[NRG][NS][6];  // internal energy of species k per density: R (c0-1), R c1/2, ..., R c4/5, R Ect
+  double g2[NRG][NA][7];  // log2(e) times: c0, -c1/2, -c2/6, -c3/12, -c4/20, c5, -c6
   double bf2[NR][2], ef2[NR][2];  // log2(e) times the Arrhenius exponents
   double troe[NR][3];            // log10 Fc, ac, an
   double rM6[NS], M6[NS], RF[NS];  // 1e-6 / M, 1e6 M, R c5 (the formation term of update_Et)
@@ -66,21 +67,18 @@ struct Fast {
 };
 __constant__ Fast cM;
 
-// true when the loaded tables fit the step (beyond mech_match's structure)
-inline bool usable(const DevConst& c) { return c.realgas != 0 && c.n_tct >= 1 && c.n_tct <= MAX_RANGES; }
-
 static inline cudaError_t setup(const DevConst& c) {
   Fast f{};
   const long double l2e = 1.0L / std::log(2.0L);
   for (int k = 0; k < NS; k++) {
     for (int j = 0; j < c.n_tct; j++) {
       const double* a = c.cf[k][j];
-      f.e6[k][j][0] = (double)(((long double)a[0] - 1.0L) * c.Ri[k]);
-      for (int m = 1; m < 5; m++) f.e6[k][j][m] = (double)((long double)a[m] * c.Ri[k] / (m + 1));
-      f.e6[k][j][5] = (double)((long double)a[7] * c.Ri[k]);
+      f.e6[j][k][0] = (double)(((long double)a[0] - 1.0L) * c.Ri[k]);
+      for (int m = 1; m < 5; m++) f.e6[j][k][m] = (double)((long double)a[m] * c.Ri[k] / (m + 1));
+      f.e6[j][k][5] = (double)((long double)a[7] * c.Ri[k]);
       if (k < NA) {
         const long double w[7] = {1.0L, -1.0L / 2, -1.0L / 6, -1.0L / 12, -1.0L / 20, 1.0L, -1.0L};
-        for (int m = 0; m < 7; m++) f.g2[k][j][m] = (double)(l2e * w[m] * a[m]);
+        for (int m = 0; m < 7; m++) f.g2[j][k][m] = (double)(l2e * w[m] * a[m]);
       }
     }
     // e = e(tm) + cv(tm) (T - tm) and g = h(tm) + cp(tm) (T - tm) - T (s(tm) + cp(tm) ln(T / tm))
@@ -90,12 +88,15 @@ static inline cudaError_t setup(const DevConst& c) {
     const long double cp = a[0] + a[1] * tm + a[2] * t2 + a[3] * t3 + a[4] * t4;
     const long double h = a[0] * tm + a[1] * t2 / 2 + a[2] * t3 / 3 + a[3] * t4 / 4 + a[4] * t5 / 5;
     const long double sm = a[0] * l + a[1] * tm + a[2] * t2 / 2 + a[3] * t3 / 3 + a[4] * t4 / 4 + a[6];
-    f.e6[k][c.n_tct][0] = (double)((cp - 1.0L) * c.Ri[k]);
-    f.e6[k][c.n_tct][5] = (double)((h - cp * tm + a[7]) * c.Ri[k]);
+    f.e6[c.n_tct][k][0] = (double)((cp - 1.0L) * c.Ri[k]);
+    f.e6[c.n_tct][k][5] = (double)((h - cp * tm + a[7]) * c.Ri[k]);
+    if (c.realgas == 0)  // e = 5/2 R T at any temperature; the equilibrium constants keep the fits
+      for (int j = 0; j < NRG; j++)
+        for (int m = 0; m < 6; m++) f.e6[j][k][m] = m == 0 ? 2.5 * c.Ri[k] : 0.0;
     if (k < NA) {
-      f.g2[k][c.n_tct][0] = (double)(l2e * cp);
-      f.g2[k][c.n_tct][5] = (double)(l2e * (h + a[5] - cp * tm));
-      f.g2[k][c.n_tct][6] = (double)(-l2e * (sm - cp * l));
+      f.g2[c.n_tct][k][0] = (double)(l2e * cp);
+      f.g2[c.n_tct][k][5] = (double)(l2e * (h + a[5] - cp * tm));
+      f.g2[c.n_tct][k][6] = (double)(-l2e * (sm - cp * l));
     }
   }
   for (int j = 0; j < NR; j++) {
@@ -141,7 +142,7 @@ struct EnergyPoly {
 #pragma unroll
     for (int k = 0; k < NS; k++)
 #pragma unroll
-      for (int m = 0; m < 6; m++) a[m] = fma(cM.e6[k][j][m], d[k], a[m]);
+      for (int m = 0; m < 6; m++) a[m] = fma(cM.e6[j][k][m], d[k], a[m]);
   }
   __device__ __forceinline__ double e(double T) const {
     return fma(T, fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]), a[5]);
@@ -325,7 +326,7 @@ __device__ __forceinline__ bool fast_step(double* di, double& E, double dt, doub
       const double l1 = 1.0 - lt;
 #pragma unroll
       for (int i = 0; i < NA; i++) {
-        const double* g = cM.g2[i][jc];
+        const double* g = cM.g2[jc][i];
         G[i] = fma(T, fma(T, fma(T, fma(T, g[4], g[3]), g[2]), g[1]), fma(g[0], l1, fma(g[5], rT, g[6])));
       }
     }

@@ -52,12 +52,23 @@ def states(kind, n):
         di[:, [names.index(s) for s in ("O", "OH", "H", "HO2", "H2O2")]] += 1e-2 * di.sum(axis=1, keepdims=True)
         dt, nsub = np.full(n, 2.0e-7), np.full(n, 2, dtype=np.int32)
         T = rng.uniform(1900.0, 2500.0, n)
+    elif kind == "ranges":  # five fit ranges
+        T = rng.uniform(400.0, 3000.0, n)
+        for k in range(9):
+            old = [list(th.coef[k][j]) for j in (0, 1)]
+            for j, o in enumerate((0, 0, 1, 1, 1)):
+                th.coef[k][j][:] = old[o]
+                th.coef[k][j][0] = old[o][0] * (1.0 + 0.01 * j)
+        th.n_tct = 5
+        th.tct[:4] = [600.0, 1000.0, 1500.0, 2200.0]
     e = np.ascontiguousarray(cases.energy_realgas(th, di.T.copy(), T))
+    if kind == "ideal":
+        e = np.ascontiguousarray(2.5 * T * (di @ np.array([8.314 / th.mi[k] for k in range(9)])))
     return th, kin, np.ascontiguousarray(di), e, np.ascontiguousarray(dt), np.ascontiguousarray(nsub)
 
 
 CASES = [("usual", 1), ("usual", 33), ("usual", 4097), ("cold", 40), ("boundary", 97), ("stiff", 65),
-         ("limit", 41), ("hot", 65), ("pivots", 321), ("overshoot", 66)]
+         ("limit", 41), ("hot", 65), ("pivots", 321), ("overshoot", 66), ("ranges", 67), ("ideal", 68)]
 
 
 def multipliers(oracle, th, kin, di, e, h):
@@ -149,7 +160,7 @@ def child(out):
     for kind, n in CASES:
         for cp in (0, 1):
             th, kin, di, e, dt, nsub = states(kind, n)
-            solver.chem_setup(th, kin, 1, abi.CHEM_IMPLICIT, const_p=bool(cp))
+            solver.chem_setup(th, kin, int(kind != "ideal"), abi.CHEM_IMPLICIT, const_p=bool(cp))
             assert solver.VARIANT == "fma" and solver.lib().ocfd_gpu_chem_compiled_mechanism(-1) == 1
             solver.chem_batch(di, e, dt, nsub)
             res["%s_%d_%d_di" % (kind, n, cp)] = di
@@ -170,7 +181,7 @@ def gpu_results(tmp_path_factory):
 def test_compiled_mechanism_step(oracle, gpu_results, kind, n, cp):
     th, kin, di, e, dt, nsub = states(kind, n)
     d0 = di.copy()
-    oracle.chem_batch(th, kin, 1, -1, di, e, dt, nsub, const_p=bool(cp))
+    oracle.chem_batch(th, kin, int(kind != "ideal"), -1, di, e, dt, nsub, const_p=bool(cp))
     gd, ge = (gpu_results["%s_%d_%d_%s" % (kind, n, cp, f)] for f in ("di", "e"))
     assert np.isfinite(di).all()
     assert (np.abs(gd - di).max(axis=1) <= 1e-10 * np.abs(di).max(axis=1)).all()
