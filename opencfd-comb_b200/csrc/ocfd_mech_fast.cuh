@@ -55,6 +55,18 @@ constexpr bool inert_last() {
   return true;
 }
 static_assert(inert_last(), "the last species takes part in no reaction");
+// O and H atoms of the species in the order that fast_step's potentials assume: O, O2, H2, H2O, OH, H, HO2, H2O2
+constexpr int ATOMS[NA][2] = {{1, 0}, {2, 0}, {0, 2}, {1, 2}, {1, 1}, {0, 1}, {2, 1}, {2, 2}};
+constexpr bool conserves_atoms() {
+  for (int j = 0; j < NR; j++)
+    for (int e = 0; e < 2; e++) {
+      int t = 0;
+      for (int i = 0; i < NA; i++) t += (VR[j][i] - VF[j][i]) * ATOMS[i][e];
+      if (t != 0) return false;
+    }
+  return true;
+}
+static_assert(conserves_atoms(), "the elements' potentials cancel in every reaction");
 
 struct Fast {
   // by fit range, so that the range in use is one stretch of the constant cache
