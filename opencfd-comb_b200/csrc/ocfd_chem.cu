@@ -31,14 +31,6 @@ cudaError_t mech_setup(const DevConst& c) {
   return cudaSuccess;
 }
 
-#ifdef OCFD_FEW_SPECIES
-#define NS_CASES(...)                                          \
-  switch (ns) {                                                \
-    case 2: { constexpr int NSV = 2; __VA_ARGS__; } break;     \
-    case 9: { constexpr int NSV = 9; __VA_ARGS__; } break;     \
-    default: throw std::runtime_error("N_SPEC must be 1..9");  \
-  }
-#else
 #define NS_CASES(...)                                          \
   switch (ns) {                                                \
     case 1: { constexpr int NSV = 1; __VA_ARGS__; } break;     \
@@ -52,7 +44,6 @@ cudaError_t mech_setup(const DevConst& c) {
     case 9: { constexpr int NSV = 9; __VA_ARGS__; } break;     \
     default: throw std::runtime_error("N_SPEC must be 1..9");  \
   }
-#endif
 
 void launch_chem_cells(int ns, long long ncell, double* f, double* Et, double* T, double* p, double* di, double dt2,
                        int nsub, int* nfail, cudaStream_t st) {
