@@ -305,7 +305,8 @@ int ocfd_gpu_ana_average(int upload, double* fields, int* k_average, double* t_a
  * the species chain (species sweeps, then divergence and RK update) runs on a third stream beside
  * the species viscous fluxes and the flow part instead of in order}. Shapes (cells along the
  * sweep x pencils): x 56x4, 120x2, 24x8; y / z 24x16, 24x8, 56x8. Every choice gives
- * bit-identical results.
+ * bit-identical results, but for the metric forms of the flux sweeps and of the viscous-flux kernel in
+ * the contracted build, which differ by rounding.
  * ocfd_gpu_autotune times each candidate on the current state (after ocfd_gpu_init_state) over reps
  * launches, applies the fastest and remembers it for this configuration (grid, schemes, species)
  * in the process; reps = 0 applies a remembered choice without timing when there is one. choice
@@ -315,7 +316,7 @@ int ocfd_gpu_ana_average(int upload, double* fields, int* k_average, double* t_a
  * best tiles: flux x, y, z, k_visc_ev, k_visc_div, then the flow right-hand side of a stage with
  * the viscous flux after and beside the flux sweeps, then a stage's right-hand sides without the
  * species RK update with the species chain in order and on the third stream (-1 where not timed).
- * The launches write only scratch arrays, so the solution is unchanged. The tuner also times the
+ * The launches write only scratch arrays, so the state is unchanged. The tuner also times the
  * per-cell k_visc_ev (not among the 27 times) and takes the per-cell pair of viscous kernels or the
  * marching pair, whichever is faster together. Default choice {0, 0, 0, 16, 0, 0, 0, 0, 3}. */
 int ocfd_gpu_autotune(int reps, int* choice, double* ms);

@@ -705,10 +705,12 @@ void chem_t(double dt2, int nsub) {
 // ---------------------------------------------------------------- stencil tile autotuner
 // Tile choices {flux x, y, z shape; k_visc_ev, k_visc_div k planes per block (0 for k_visc_div: both
 // kernels in their per-cell forms); metric form of the flux sweeps, k_visc_ev, k_visc_div; k_visc_ev
-// beside the flux sweeps on a second stream or after them}. Every choice gives bit-identical results (a tile decides
-// which block computes a point, not how; the stored metric arrays hold the values the separable
-// form computes), so the tuner is free to pick by time alone. Choices are remembered per
-// configuration in the process.
+// beside the flux sweeps on a second stream or after them}. In the exact build every choice gives
+// bit-identical results (a tile decides which block computes a point, not how; the stored metric arrays
+// hold the values the separable form computes). In the contracted build that holds for all but the metric
+// forms of the flux sweeps and of k_visc_ev: the separable form leaves out divisions and, along one grid
+// direction, the zeros of the metric, so the stored form differs from it by rounding. The tuner picks by
+// time alone in both. Choices are remembered per configuration in the process.
 constexpr int TUNE_N = 9, TUNE_TIMES = 3 * FLUX_TILE_SHAPES + 9 + 5 + 2 + 2;
 std::map<std::string, std::array<int, TUNE_N>> g_tune_cache;
 

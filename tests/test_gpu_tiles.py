@@ -1,9 +1,15 @@
 """Stencil tile autotuner: every tile shape of the flow-flux sweeps and every k-chunk of the
 marching viscous kernels gives bit-identical states (a tile decides which block computes a point,
 not how), and the tuner's timed choice is one of the candidates and leaves the solution unchanged."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
+if __name__ == "__main__":  # the child of the contracted build's tests
+    sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "opencfd-comb_b200"))
 from ocfd_b200 import abi, cases, solver
 
 pytestmark = pytest.mark.gpu
@@ -130,3 +136,48 @@ def test_reported_tiles_are_those_that_run(tuned):
     assert ms() < 1.8 * before
     g.profile(False)
     g.close()
+
+
+STORED = [[0, 0, 0, 16, 0, 1, 0, 0, 0], [0, 0, 0, 16, 0, 0, 1, 0, 3], [1, 2, 0, 8, 16, 1, 1, 1, 1]]
+
+
+def _child(out):
+    """every choice on every case in this process's library"""
+    res = {"variant": solver.VARIANT}
+    for kind in ("flatplate", "isotropic", "jet"):
+        c = _case(kind)
+        plain = [c2[:5] + [0, 0, c2[7]] + c2[8:] for c2 in CHOICES]
+        for n, choice in enumerate([None] + plain + STORED):
+            st, _ = _run(c, choice)
+            for m, a in enumerate(st):
+                res["%s_%d_%d" % (kind, n, m)] = a
+    np.savez(out, **res)
+
+
+@pytest.fixture(scope="module")
+def contracted(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("tiles") / "gpu.npz")
+    subprocess.run([sys.executable, os.path.abspath(__file__), out], check=True, timeout=300,
+                   env=dict(os.environ, OCFD_B200_LIB="fma"))
+    return np.load(out)
+
+
+@pytest.mark.parametrize("kind", ["flatplate", "isotropic", "jet"])
+def test_tile_choices_in_the_contracted_build(contracted, kind):
+    """all choices with the computed metrics of the flux sweeps and the viscous-flux kernel are
+    bit-identical; with the stored ones the conserved fields agree to the build's 1e-10 (a momentum
+    component of the plate cancels to a small part of the largest: 1e-13 of that on top)"""
+    assert str(contracted["variant"]) == "fma"
+    ref = [contracted["%s_0_%d" % (kind, m)] for m in range(3)]
+    for n in range(1, 1 + len(CHOICES)):
+        for m in range(3):
+            assert np.array_equal(contracted["%s_%d_%d" % (kind, n, m)], ref[m]), n
+    mom = 1e-13 * np.abs(ref[0][1:4]).max()
+    for n in range(1 + len(CHOICES), 1 + len(CHOICES) + len(STORED)):
+        f = contracted["%s_%d_0" % (kind, n)]
+        for m in range(5):
+            assert np.abs(f[m] - ref[0][m]).max() <= 1e-10 * np.abs(ref[0][m]).max() + mom * (1 <= m <= 3), (n, m)
+
+
+if __name__ == "__main__":
+    _child(sys.argv[1])
