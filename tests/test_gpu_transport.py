@@ -1,5 +1,5 @@
 """Fitted mixture transport (k_transport_fit) against the CPU oracle for every species count's
-dispatch. The viscosity is compared as the mean that ana_box reports; conductivity and diffusion
+dispatch and both library builds. The viscosity is compared as the mean that ana_box reports; conductivity and diffusion
 through what they do to the state: the difference of a viscous and an inviscid step, which is the
 viscous terms alone.
 
@@ -7,9 +7,15 @@ Tolerances: the coefficients are products of exponentials with a few ulp each, s
 agrees to 1e-12. In the step differences the states' own rounding (a few hundred operations, 1e-13
 of the largest value) stands against the viscous increment; 1e-10 of the increment is allowed on top.
 """
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
+if __name__ == "__main__":  # the child of the contracted build's test
+    sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "opencfd-comb_b200"))
 from ocfd_b200 import cases, solver
 
 pytestmark = pytest.mark.gpu
@@ -76,3 +82,46 @@ def test_cells_of_one_species(oracle, ns):
         for m in range(len(r)):
             want, got = r[m] - s[m], a[m] - b[m]
             assert np.abs(got - want).max() <= 1e-13 * np.abs(r[m]).max() + 1e-10 * np.abs(want).max(), m
+
+
+ALL = [(2, 9), (3, 8), (4, 10), (5, 13), (6, 9), (7, 12), (8, 8), (9, 11)]
+UNMIXED = [2, 9]
+
+
+def _child(out):
+    res = {"variant": solver.VARIANT}
+    for tag, c in [("t%d" % ns, case(n, ns, ns)) for ns, n in ALL] + [("u%d" % ns, unmixed(ns)) for ns in UNMIXED]:
+        for v, (f, di, mu) in enumerate(steps(solver.Solver, c)):
+            res["%s_f%d" % (tag, v)], res["%s_d%d" % (tag, v)] = f, di
+            if mu is not None:
+                res[tag + "_mu"] = mu
+    np.savez(out, **res)
+
+
+@pytest.fixture(scope="module", params=["exact", "fma"])
+def both_builds(request, tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("transport") / "gpu.npz")
+    subprocess.run([sys.executable, os.path.abspath(__file__), out], check=True, timeout=300,
+                   env=dict(os.environ, OCFD_B200_LIB=request.param))
+    z = np.load(out)
+    assert str(z["variant"]) == request.param
+    return z
+
+
+@pytest.mark.parametrize("tag,make", [("t%d" % ns, (lambda ns=ns, n=n: case(n, ns, ns))) for ns, n in ALL] +
+                         [("u%d" % ns, (lambda ns=ns: unmixed(ns))) for ns in UNMIXED])
+def test_every_species_count_in_both_builds(oracle, both_builds, tag, make):
+    """the same comparison and bounds for every instance of the kernel in the exact and the contracted
+    library; the contracted flow kernels' own rounding is that of the states, 1e-13 of the largest value"""
+    ov, oi = steps(oracle.OracleSolver, make())
+    if tag[0] == "t":
+        assert abs(both_builds[tag + "_mu"] - ov[2]) <= 1e-12 * abs(ov[2])
+    for k, v in (("f", 0), ("d", 1)):
+        for m in range(len(ov[v])):
+            want = ov[v][m] - oi[v][m]
+            got = both_builds["%s_%s0" % (tag, k)][m] - both_builds["%s_%s1" % (tag, k)][m]
+            assert np.abs(got - want).max() <= 1e-13 * np.abs(ov[v][m]).max() + 1e-10 * np.abs(want).max(), (k, m)
+
+
+if __name__ == "__main__":
+    _child(sys.argv[1])
