@@ -541,7 +541,7 @@ __device__ __forceinline__ void dev_diffusion(double* amd, double amu, double T,
 // operations per reconstruction instead of the 52 of the term-by-term form with one division. The
 // same quantities up to rounding; the products stay in range while the split fluxes are below about
 // 1e30. The sweeps issue FP64 and shared-memory instructions at 60-75 % of the issue rate, so the
-// count is the time: the species sweeps of the 384x256x32 jet 11.7 -> 7.85 ms per step, the flow
+// count is the time: the species sweeps of the 384x256x32 jet 11.7 -> 7.94 ms per step, the flow
 // sweeps x / y / z 1.50 / 1.66 / 2.68 -> 1.26 / 1.40 / 1.95; 64^3 box 0.20 / 0.20 / 0.21 -> 0.17 /
 // 0.17 / 0.18.
 __device__ __forceinline__ double w5D(double s) { return fma(13.0 / 3.0 * s, s, 4.0e-6); }

@@ -1027,11 +1027,11 @@ __global__ void __launch_bounds__(VE_THREADS, 2) k_visc_div(DivArgs a) {
 // resident-block target of the per-cell k_visc_div: it waits on its stencil loads; ten blocks of 128
 // threads (48 registers) against eight / twelve: 1.126 against 1.158 / 1.098 ms per step on the
 // 384x256x32 jet, 0.201 against 0.223 / 0.210 on 97x61x43, 1.55 against 1.55 / 1.58 on 1024x160x32.
-// In 32 x 4 tiles of cells: on those grids 1.69 (marching, 16 planes), 0.52 and 2.37 ms per step
+// The marching form at its default 16 planes takes 1.69, 0.52 and 2.37 ms on those grids.
 #ifndef OCFD_VDIV_MINB
 #define OCFD_VDIV_MINB 10
 #endif
-// per-cell form of k_visc_div (the autotuner's k chunk 0): one thread per cell, every stencil
+// per-cell form of k_visc_div (choice[4] = 0): one thread per cell, every stencil
 // value read through the read-only cache; the same expressions as the marching form
 template <bool SEP, int HZ>
 __global__ void __launch_bounds__(32 * PC_TY, OCFD_VDIV_MINB) k_visc_div_pc(DivArgs a, int nbx) {

@@ -73,7 +73,7 @@ __device__ __forceinline__ double cubic(const double* c, double L) {
 // exponentials of 12, the Wilke quadratics 243). The form it replaces spread a cell over one thread
 // per species with nine barriers' worth of shared-memory exchange: 9250 issued instructions per cell,
 // 2400 of them FP64, at 27 % of the FP64 pipe. Measured on 384x256x32 cells, 9 species (contracted
-// build): 1.540 -> 0.305 ms per launch, about 80 % of the measured FP64 rate; 97x61x43: 0.140 -> 0.034.
+// build): 1.540 -> 0.303 ms per launch, 75 % of the FP64 pipe; 97x61x43: 0.140 -> 0.033.
 // 128 threads x 4 blocks leave 128 registers, which hold it without spills.
 #ifndef OCFD_TFIT_THREADS
 #define OCFD_TFIT_THREADS 128
