@@ -73,7 +73,7 @@ __device__ __forceinline__ double cubic(const double* c, double L) {
 // exponentials of 12, the Wilke quadratics 243). The form it replaces spread a cell over one thread
 // per species with nine barriers' worth of shared-memory exchange: 9250 issued instructions per cell,
 // 2400 of them FP64, at 27 % of the FP64 pipe. Measured on 384x256x32 cells, 9 species (contracted
-// build): 1.540 -> 0.303 ms per launch, 75 % of the FP64 pipe; 97x61x43: 0.140 -> 0.033.
+// build): 1.540 -> 0.294 ms per launch, three quarters of the FP64 pipe; 97x61x43: 0.140 -> 0.033.
 // 128 threads x 4 blocks leave 128 registers, which hold it without spills.
 #ifndef OCFD_TFIT_THREADS
 #define OCFD_TFIT_THREADS 128
@@ -99,22 +99,17 @@ __global__ void __launch_bounds__(OCFD_TFIT_THREADS, OCFD_TFIT_MINB)
   double X0 = 0.0;
 #pragma unroll
   for (int m = 0; m < NS; m++) {
-    X[m] = di[(size_t)m * cC.H + q] * cF.rMi[m];
+    X[m] = __dmul_rn(di[(size_t)m * cC.H + q], cF.rMi[m]);
     X0 += X[m];
   }
-  // mole fractions: the product with 1 / X0 and its remainder, so that a cell of one species alone gets
-  // X = 1 exactly, as the division gives it. Its 1 - X is then 0; one unit in the last place of X
-  // instead would be divided by ds = 1e-20 below.
-  const double rX = rcp3(X0);
-#pragma unroll
-  for (int m = 0; m < NS; m++) {
-    const double x = X[m] * rX;
-    X[m] = fma(fma(-x, X0, X[m]), rX, x);
-  }
+  // Mole numbers take the mole fractions' place; their sum X0 enters where it does not cancel. Thereby
+  // 1 - X_k is (X0 - X[k]) / X0, which is 0 where a species is alone, as with the reference's quotient; a
+  // rounded product with 1 / X0 would leave one unit in the last place there, to be divided by 1e-20. (Of
+  // rounded products, not contracted: X0 then equals X[k] beside traces below its last place as well.)
   // diffusion: ds_k = sum over j != k of X_j / D_kj, every pair's exponential once
   double ds[NS];
 #pragma unroll
-  for (int m = 0; m < NS; m++) ds[m] = 1.0e-20;
+  for (int m = 0; m < NS; m++) ds[m] = 1.0e-20 * X0;
   {
     int np = 0;
 #pragma unroll
@@ -127,7 +122,7 @@ __global__ void __launch_bounds__(OCFD_TFIT_THREADS, OCFD_TFIT_MINB)
       }
   }
 #pragma unroll
-  for (int m = 0; m < NS; m++) amd[(size_t)m * cC.N + t] = (1.0 - X[m]) * rp * rcp3(ds[m]);
+  for (int m = 0; m < NS; m++) amd[(size_t)m * cC.N + t] = (X0 - X[m]) * rp * rcp3(ds[m]);
   // conductivity: mean of the arithmetic and harmonic means
   {
     double a1 = 0.0, a2 = 0.0;
@@ -137,7 +132,7 @@ __global__ void __launch_bounds__(OCFD_TFIT_THREADS, OCFD_TFIT_MINB)
       a1 = fma(X[m], kk, a1);
       a2 = fma(X[m], rcp3(kk), a2);
     }
-    amk[t] = 0.5 * (a1 + rcp3(a2));
+    amk[t] = 0.5 * fma(a1, rcp3(X0), X0 * rcp3(a2));
   }
   // viscosity: mu = sum_k X_k mu_k / sum_j X_j phi_kj
   double s[NS], Y[NS], Z[NS];  // sqrt(mu_k), X_k / s_k, X_k / mu_k

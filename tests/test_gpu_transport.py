@@ -60,13 +60,14 @@ def test_transport_fit_against_oracle(oracle, ns, n):
             assert np.abs(got - want).max() <= 1e-13 * np.abs(r[m]).max() + 1e-10 * np.abs(want).max(), m
 
 
-def unmixed(ns, n=12):
-    """two of the species side by side, each alone in its half of a periodic box"""
+def unmixed(ns, n=12, trace=0.0):
+    """two of the species side by side, each alone in its half of a periodic box, but for traces of all"""
     c = case(n, ns, ns)
     half = np.where(np.arange(n) < n // 2, 1.0, 0.0)
     d = c.di.sum(axis=0)
-    c.di = np.zeros_like(c.di)
-    c.di[0], c.di[1] = d * half, d * (1.0 - half)
+    c.di = np.zeros_like(c.di) + trace * d
+    c.di[0] += d * half
+    c.di[1] += d * (1.0 - half)
     return c
 
 
@@ -85,12 +86,15 @@ def test_cells_of_one_species(oracle, ns):
 
 
 ALL = [(2, 9), (3, 8), (4, 10), (5, 13), (6, 9), (7, 12), (8, 8), (9, 11)]
-UNMIXED = [2, 9]
+CASES = [("t%d" % ns, (lambda ns=ns, n=n: case(n, ns, ns))) for ns, n in ALL]
+CASES += [("u%d" % ns, (lambda ns=ns: unmixed(ns))) for ns in (2, 9)]
+CASES += [("v%d" % ns, (lambda ns=ns: unmixed(ns, trace=1.0e-18))) for ns in (2, 9)]
 
 
 def _child(out):
     res = {"variant": solver.VARIANT}
-    for tag, c in [("t%d" % ns, case(n, ns, ns)) for ns, n in ALL] + [("u%d" % ns, unmixed(ns)) for ns in UNMIXED]:
+    for tag, make in CASES:
+        c = make()
         for v, (f, di, mu) in enumerate(steps(solver.Solver, c)):
             res["%s_f%d" % (tag, v)], res["%s_d%d" % (tag, v)] = f, di
             if mu is not None:
@@ -108,8 +112,7 @@ def both_builds(request, tmp_path_factory):
     return z
 
 
-@pytest.mark.parametrize("tag,make", [("t%d" % ns, (lambda ns=ns, n=n: case(n, ns, ns))) for ns, n in ALL] +
-                         [("u%d" % ns, (lambda ns=ns: unmixed(ns))) for ns in UNMIXED])
+@pytest.mark.parametrize("tag,make", CASES, ids=[tag for tag, _ in CASES])
 def test_every_species_count_in_both_builds(oracle, both_builds, tag, make):
     """the same comparison and bounds for every instance of the kernel in the exact and the contracted
     library; the contracted flow kernels' own rounding is that of the states, 1e-13 of the largest value"""
