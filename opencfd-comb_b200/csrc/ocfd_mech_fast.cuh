@@ -14,18 +14,18 @@
 // more fit range here, so that hot reactors, and Newton's first guesses beyond it, take the same path.
 // What is left, T below T_MIN or no T(E), takes the sub-step of chem_step<9, ..., MECH_H2AIR9>, its
 // matrix in the block's shared memory.
-// Bound by FP64 issue and its latency at eight warps per SM (212 registers, more than half of them the
+// Bound by FP64 issue and its latency at eight warps per SM (254 registers with its callees, half of them the
 // 8 x 8 matrix; the rates of progress wait in shared memory until it is assembled, so the two phases'
 // values are not live together). About 1500 FP64 operations per sub-step against some 3500 with the
 // matrix in shared memory, 42 equilibrium and rate exponentials of 20, and a division per pivot row.
-// Measured against that form (k_chem_batch): 2^20 reactors with 22 sub-steps on average 20.7 -> 4.60 ms
-// (0.88 -> 0.20 ns per sub-step), 60,001 at constant pressure 4.13 -> 0.91 ms, the cells of the
+// Measured against that form (k_chem_batch): 2^20 reactors with 22 sub-steps on average 20.9 -> 4.51 ms
+// (0.88 -> 0.19 ns per sub-step), 60,001 at constant pressure 4.11 -> 0.90 ms, the cells of the
 // 384x256x32 jet 3.19 -> 0.72 ms per step. 777 reactors on host arrays, up to a hundred sub-steps in a row
-// on one thread each, whole call 3.9 -> 0.60 ms: the step's latency is below the cooperative kernel's, so
+// on one thread each, whole call 3.8 -> 0.58 ms: the step's latency is below the cooperative kernel's, so
 // batches of every size come here. 2^18 reactors, 20 sub-steps, at 300-400 K / 100-148 K / steam at
-// 2500-4000 K / products at 5100-6500 K: 4.90 / 4.90 / 5.06 / 5.75 -> 1.25 / 1.25 / 1.34 / 1.46 ms. With steps
+// 2500-4000 K / products at 5100-6500 K: 4.90 / 4.90 / 5.06 / 5.75 -> 1.24 / 1.25 / 1.30 / 1.37 ms. With steps
 // so long that densities overshoot below zero (1e-7 s, a hundredth of radicals) 1.15 -> 0.57, with one
-// reactor in sixty lost (1e-6 s) 2.28 -> 2.12. Below T_MIN the step is the same and slower than in its own
+// reactor in sixty lost (1e-6 s) 2.28 -> 2.06. Below T_MIN the step is the same and slower than in its own
 // kernel (85-99 K, one lane in three: 4.90 -> 7.9).
 #pragma once
 #include "ocfd_chem.cuh"

@@ -16,8 +16,9 @@ namespace ocfd {
 // 3 TB/s of DRAM traffic. More warps per SM are slower, not faster: at 96 / 72 registers instead of
 // 128 the pair of kernels took 8.3 instead of 6.8 ms per jet step, their rows evicting one another
 // from L1; fewer (168 registers) 7.3; cp.async staging of the planes 8.1; two planes per thread 7.7.
-// Measured with k_ci and the face cells, 9 species, contracted build: 384x256x32 10.2 -> 6.75 ms per
-// step, 97x61x43 1.13 -> 0.85.
+// Measured with k_ci and the face cells, 9 species, ms per step, CD6 / CD8: contracted build 384x256x32
+// 10.3 / 11.1 -> 6.8 / 7.6, 97x61x43 1.13 / 1.20 -> 0.85 / 0.94; exact build, whose face cells are three or
+// four layers deep, 11.2 / 12.1 -> 7.7 / 8.7 and 1.21 / 1.30 -> 0.97 / 1.07.
 constexpr int SV_TY = 4, SV_SLAB = 32 / SV_TY;
 #ifndef OCFD_SE_MINB
 #define OCFD_SE_MINB 4
